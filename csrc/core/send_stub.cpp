@@ -272,7 +272,12 @@ struct KvSendStub::Impl {
     const bool whole = batch.step->frozen && ch->send_layers(start_layer, num_layers, batch.step.get());
     for (uint32_t i = start_layer; i < num_layers && !whole;) {
       TimeWatch w;
-      if (by_record) batch.step->wait_layer_recorded(i); else batch.step->wait_layer_ready(i);
+      if (by_record) {
+        const size_t rem = num_layers - i, want = std::min(std::max<size_t>(1, ch->preferred_run(rem)), rem);
+        batch.step->wait_layer_recorded(i + static_cast<uint32_t>(want) - 1);
+      } else {
+        batch.step->wait_layer_ready(i);
+      }
       pb.wait_us += w.get_elapse_us();
       if (by_record) {
         // layers recorded while the sender was busy go out together where the channel can do that

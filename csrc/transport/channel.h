@@ -38,6 +38,12 @@ class IChannel {
     (void)layer_begin; (void)layer_end; (void)step;
     return false;
   }
+  // With `remaining` layers of the batch still to send: how many the channel would like to be recorded before the next
+  // send_range() (device ordered transports only).  A launch can then carry several.
+  virtual size_t preferred_run(size_t remaining) const {
+    (void)remaining;
+    return 1;
+  }
   // Layers [layer_begin, layer_end) are all ready (device ordered: all recorded).  Sends the first one
   // or, when one launch can carry several, the first few; returns how many it took (>= 1).
   virtual size_t send_range(size_t layer_begin, size_t layer_end, Step* step) {

@@ -1,0 +1,78 @@
+"""Several layers of a step in one launch: whatever the launches hold, every layer's bytes are those that the forward stream wrote
+before it recorded the layer's event, and nothing outside the request's slots is written."""
+import os
+import time
+
+import pytest
+import torch
+
+os.environ.setdefault("BLLM_KVTRANS_QUIET_ENV", "1")
+
+from llumnix_kv_b200.kv_transfer_impl import KVTransferClient, KVTransferProtocolType as PT, KVTransferServer
+from llumnix_kv_b200.ops.layouts import AttnLayout, CacheShape
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+BLOCK = 64
+
+
+class _Cache:
+    """One rank's cache of a shape: its tensors, the sizes that the engine is told, and a request's bytes of a layer."""
+
+    def __init__(self, shape, layers, blocks):
+        self.mla = shape == CacheShape.DPSK_V32_SPARSE_MLA
+        self.lay = AttnLayout(CacheShape.FLASH, blocks, BLOCK, 8, 128, 2)
+        self.toks = [132, 656] if self.mla else [self.lay.token_bytes]
+        self.layers = [[torch.zeros(blocks * BLOCK * t, dtype=torch.uint8, device=DEV) for t in self.toks] for _ in range(layers)]
+        one = (lambda x: x) if self.mla else (lambda x: x[0])
+        self.args = one([BLOCK * t for t in self.toks]), one(self.toks), "fake://", [one(t) for t in self.layers], [PT.NVLINK]
+        self.kw = dict(num_kv_heads=1 if self.mla else 8, cache_shape=int(shape))
+
+    def rows(self, layer, first, n):
+        """Every token slot of blocks [first, first + n), one row each and tensor."""
+        if not self.mla:
+            v = self.lay.view(self.layers[layer][0], torch.int16)[first:first + n]     # [block, kv, slot, head, dim]
+            return [v.movedim(1, 2).reshape(n * BLOCK, -1).view(torch.uint8)]
+        return [t.view(-1, BLOCK * k)[first:first + n].reshape(n * BLOCK, k) for t, k in zip(self.layers[layer], self.toks)]
+
+
+@pytest.mark.parametrize("host_gap_s", [0.0, 0.002])
+@pytest.mark.parametrize("shape", [CacheShape.FLASH, CacheShape.DPSK_V32_SPARSE_MLA])
+@pytest.mark.parametrize("layers, tokens", [(1, 16), (2, 1), (13, 75), (13, 3001), (33, 700)])
+def test_every_layer_carries_what_was_recorded(layers, tokens, shape, host_gap_s):
+    """75 tokens: 4 MiB hold every layer.  3001: a quarter of the rest per launch.  host_gap_s: a forward thread slower than the
+    sender, so that it waits for layers; without it the layers are all recorded long before the GPU has produced them."""
+    n = -(-tokens // BLOCK)
+    src, dst = _Cache(shape, layers, 2 * n + 2), _Cache(shape, layers, 2 * n + 2)
+    srv = KVTransferServer("D|0|1", 1, 0, 0, *dst.args, **dst.kw)
+    cli = KVTransferClient("P|0|1", 1, 0, 0, *src.args, **src.kw)
+    try:
+        fwd = torch.cuda.Stream()
+        big = torch.empty(1 << 26, dtype=torch.uint8, device=DEV)
+        for step in (1, 2, 3):
+            sb, db = list(range(1, n + 1)), list(range(n + 1, 2 * n + 1))
+            cli.submit_req_send2("D|0|1", 0, "r%d" % step, 0, tokens, True, sb, db, srv.worker_info(), stepid=step)
+            cli.start_send_step(step, 1)
+            with torch.cuda.stream(fwd):
+                for layer in range(layers):
+                    big.fill_(layer)                     # the layer is produced "late"
+                    for t in src.layers[layer]:
+                        t.fill_((7 * layer + 31 * step) % 251 + 1)
+                    cli.record_event(layer, fwd)
+                    time.sleep(host_gap_s)
+            cli.flush_send_step()
+            assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+            torch.cuda.synchronize()
+            for layer in range(layers):
+                v = (7 * layer + 31 * step) % 251 + 1
+                for got in dst.rows(layer, n + 1, n):
+                    assert int(got[:tokens].min()) == int(got[:tokens].max()) == v
+                    assert dst.mla or not bool(got[tokens:].any())
+                for untouched in dst.rows(layer, 0, n + 1):
+                    assert not bool(untouched.any())
+    finally:
+        cli.drain()
+        del cli
+        srv.stop()
