@@ -4,6 +4,8 @@
 // objects so that several workers can live in one process (tests, single-process demos).
 #include <chrono>
 
+#include <cuda_runtime.h>
+
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
@@ -183,6 +185,12 @@ std::unique_ptr<KvServer> g_server;
 KvTransferClient* need_client() {
   if (!g_client) throw KVTransferException(ErrorKind::INVALID_OPERATION, "kv client is not initialized");
   return g_client->get();
+}
+
+// One layer of the forward pass: its event on the engine's stream, and word of it to the open step.
+void record_layer(KvTransferClient* c, size_t stepid, uint64_t event, uint64_t stream) {
+  cuda_check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "cudaEventRecord(layer)");
+  c->notify_event_record(stepid);
 }
 
 std::optional<WorkerInfo> parse_py_worker_info(const py::handle& h) {
@@ -428,6 +436,8 @@ void bind_engine(py::module_& m) {
       .def("start_send", [](KvClient& c, size_t stepid, size_t sched) { return c.get()->start_send(stepid, sched); },
            py::arg("stepid") = 1024, py::arg("sched_tokens") = 1)
       .def("notify_event_record", [](KvClient& c, size_t stepid) { c.get()->notify_event_record(stepid); })
+      .def("record_layer",
+           [](KvClient& c, size_t stepid, uint64_t event, uint64_t stream) { record_layer(c.get(), stepid, event, stream); })
       .def("flush_send", [](KvClient& c, size_t stepid) { c.get()->flush_send(stepid); })
       .def("drain", [](KvClient& c) { c.get()->drain(); }, py::call_guard<py::gil_scoped_release>())
       .def("wait_inflight",
@@ -537,6 +547,7 @@ void bind_engine(py::module_& m) {
     need_client()->start_send_substep(stepid, substepid, metas);
   });
   m.def("notify_event_record", [](size_t stepid) { need_client()->notify_event_record(stepid); });
+  m.def("record_layer", [](size_t stepid, uint64_t event, uint64_t stream) { record_layer(need_client(), stepid, event, stream); });
   m.def("flush_send", [](size_t stepid) { need_client()->flush_send(stepid); });
   m.def(
       "current_worker_info",

@@ -363,6 +363,8 @@ struct KvSendStub::Impl {
     }
     bool ok = true, async = false;
     if (!pb.send_req.empty()) {
+      // said before the planning: the wait-layers thread then follows the layers from the first on
+      if (!ch || !ch->device_ordered()) batch.step->want_ready();
       try {
         try_create_channel();
         for (const ReqSendTask* t : pb.send_req)

@@ -32,8 +32,19 @@ class Step {
   explicit Step(size_t idx) : step_idx(idx) {}
   ~Step();
 
-  void wait_layer_ready(uint32_t layer) { data_signal_.wait(layer); }
-  bool wait_layer_ready_for(uint32_t layer, std::chrono::milliseconds d) { return data_signal_.wait_for(layer, d); }
+  void wait_layer_ready(uint32_t layer) { want_ready(); data_signal_.wait(layer); }
+  bool wait_layer_ready_for(uint32_t layer, std::chrono::milliseconds d) { want_ready(); return data_signal_.wait_for(layer, d); }
+  // A host-driven transport is going to follow ready(i) layer by layer.  Without it the wait-layers thread sleeps until
+  // every layer has been recorded and then waits for the last event alone: its waits for the others would contend for
+  // the driver with the forward thread's event records and the sender's launches, for nobody.
+  void want_ready() {
+    if (!ready_wanted_.exchange(true, std::memory_order_acq_rel)) record_signal_.kick();
+  }
+  // wait-layers thread: true when all `layers` have been recorded before anybody wanted ready(i)
+  bool all_recorded_unwanted(uint32_t layers) {
+    return !ready_wanted_.load(std::memory_order_acquire) && record_signal_.wait_or(layers - 1, ready_wanted_) &&
+           !ready_wanted_.load(std::memory_order_acquire);
+  }
   uint32_t notify_layer_ready(uint32_t layers_done) { return data_signal_.release(layers_done); }
   void wait_layer_recorded(uint32_t layer) { record_signal_.wait(layer); }
   uint32_t notify_layer_recorded(uint32_t layers_recorded) { return record_signal_.release(layers_recorded); }
@@ -46,6 +57,7 @@ class Step {
  private:
   SyncSemaphore data_signal_;
   SyncSemaphore record_signal_;
+  std::atomic<bool> ready_wanted_{false};
   std::atomic<int64_t> last_send_finish_{0};
 };
 

@@ -10,6 +10,7 @@
 #include <sys/socket.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
@@ -27,32 +28,60 @@ void SyncSemaphore::wait(uint32_t cond) {
 #endif
   }
   std::unique_lock<std::mutex> lk(mu_);
-  cv_.wait(lk, [&] { return ready_ > cond; });
+  while (ready_ <= cond) {
+    lowest_ = std::min(lowest_, cond);
+    cv_.wait(lk);
+  }
+}
+
+bool SyncSemaphore::wait_or(uint32_t cond, const std::atomic<bool>& other) {
+  std::unique_lock<std::mutex> lk(mu_);
+  while (ready_ <= cond && !other.load(std::memory_order_acquire)) {
+    lowest_ = std::min(lowest_, cond);
+    cv_.wait(lk);
+  }
+  return ready_ > cond;
+}
+
+void SyncSemaphore::kick() {
+  std::unique_lock<std::mutex> lk(mu_);
+  lowest_ = UINT32_MAX;
+  lk.unlock();
+  cv_.notify_all();
 }
 
 bool SyncSemaphore::wait_for(uint32_t cond, std::chrono::milliseconds timeout) {
+  const auto deadline = std::chrono::steady_clock::now() + timeout;
   std::unique_lock<std::mutex> lk(mu_);
-  return cv_.wait_for(lk, timeout, [&] { return ready_ > cond; });
+  while (ready_ <= cond) {
+    lowest_ = std::min(lowest_, cond);
+    if (cv_.wait_until(lk, deadline) == std::cv_status::timeout) return ready_ > cond;
+  }
+  return true;
+}
+
+// The counter has moved: wake the blocked waiters if it has passed the lowest of their conditions (those that it has not
+// reached enter theirs again).  The engine's forward thread releases once per layer: a wake-up for every layer of threads
+// that wait for a later one would cost it a system call each time.
+void SyncSemaphore::pass(std::unique_lock<std::mutex>& lk) {
+  fast_.store(ready_, std::memory_order_release);
+  const bool wake = ready_ > lowest_;
+  if (wake) lowest_ = UINT32_MAX;
+  lk.unlock();
+  if (wake) cv_.notify_all();
 }
 
 void SyncSemaphore::release() {
-  {
-    std::lock_guard<std::mutex> g(mu_);
-    ++ready_;
-    fast_.store(ready_, std::memory_order_release);
-  }
-  cv_.notify_all();
+  std::unique_lock<std::mutex> lk(mu_);
+  ++ready_;
+  pass(lk);
 }
 
 uint32_t SyncSemaphore::release(uint32_t cond) {
-  uint32_t v;
-  {
-    std::lock_guard<std::mutex> g(mu_);
-    if (ready_ < cond) ready_ = cond;
-    v = ready_;
-    fast_.store(ready_, std::memory_order_release);
-  }
-  cv_.notify_all();
+  std::unique_lock<std::mutex> lk(mu_);
+  if (ready_ < cond) ready_ = cond;
+  const uint32_t v = ready_;
+  pass(lk);
   return v;
 }
 

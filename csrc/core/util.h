@@ -39,15 +39,21 @@ class TimeWatch {
 class SyncSemaphore {
  public:
   void wait(uint32_t cond);
+  // As wait(), but also ends when `other` is set (by a thread that calls kick() afterwards).  True: the counter passed cond.
+  bool wait_or(uint32_t cond, const std::atomic<bool>& other);
+  void kick();
   bool wait_for(uint32_t cond, std::chrono::milliseconds timeout);
   void release();                    // counter += 1
   uint32_t release(uint32_t cond);   // counter = max(counter, cond); returns the new value
   uint32_t value();
 
  private:
+  void pass(std::unique_lock<std::mutex>& lk);
+
   alignas(64) std::mutex mu_;
   std::condition_variable cv_;
   uint32_t ready_{0};
+  uint32_t lowest_{UINT32_MAX};     // lowest condition among the blocked waiters: a release that does not pass it wakes nobody
   std::atomic<uint32_t> fast_{0};   // mirror of ready_ for the short spin before blocking
 };
 

@@ -273,6 +273,13 @@ class KVTransferClient:
         if self._cur_step_id is None:
             return  # warm-up forward passes before the first step are ignored
         if self._events:
+            # once per layer on the engine's forward thread: the raw handle of the current stream costs 0.2 us where the Stream
+            # object that Event.record() makes costs 3.5, and one native call records and notifies
+            device = torch._C._cuda_getDevice()
+            if stream is None or stream.device_index == device:
+                raw = torch._C._cuda_getCurrentRawStream(device) if stream is None else stream.cuda_stream
+                self._call("record_layer", self._cur_step_id, self._event_addrs[layer_id], raw)
+                return
             self._events[layer_id].record(stream)
         self._call("notify_event_record", self._cur_step_id)
 

@@ -76,3 +76,33 @@ def test_every_layer_carries_what_was_recorded(layers, tokens, shape, host_gap_s
         cli.drain()
         del cli
         srv.stop()
+
+
+def test_layers_recorded_on_the_current_stream_whichever_it_is():
+    """record_event() without a stream takes the current one, also when that changes from step to step."""
+    layers, n = 6, 5
+    src, dst = _Cache(CacheShape.FLASH, layers, 2 * n + 2), _Cache(CacheShape.FLASH, layers, 2 * n + 2)
+    srv = KVTransferServer("D|0|1", 1, 0, 0, *dst.args, **dst.kw)
+    cli = KVTransferClient("P|0|1", 1, 0, 0, *src.args, **src.kw)
+    try:
+        streams = [torch.cuda.Stream(), torch.cuda.default_stream(), torch.cuda.Stream()]
+        big = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+        for step in range(1, 7):
+            cli.submit_req_send2("D|0|1", 0, "r%d" % step, 0, n * BLOCK, True, list(range(n)), list(range(n + 1, 2 * n + 1)),
+                                 srv.worker_info(), stepid=step)
+            cli.start_send_step(step, 1)
+            with torch.cuda.stream(streams[step % 3]):
+                for layer in range(layers):
+                    big.fill_(layer)
+                    src.layers[layer][0].fill_(10 * step + layer)
+                    cli.record_event(layer)
+            cli.flush_send_step()
+            assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+            torch.cuda.synchronize()
+            for layer in range(layers):
+                got = dst.rows(layer, n + 1, n)[0]
+                assert int(got.min()) == int(got.max()) == 10 * step + layer
+    finally:
+        cli.drain()
+        del cli
+        srv.stop()
