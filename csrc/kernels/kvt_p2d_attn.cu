@@ -116,6 +116,39 @@ __device__ __forceinline__ bool tile_is_full(const KvtAttnLaunch& p, const TileI
   return ti.copy_lo == ti.tok_lo && ti.copy_hi == ti.tok_lo + p.tile_tokens;
 }
 
+// Work item w of a launch -> layer, K or V, tile of the layer.
+__device__ __forceinline__ void split_work(const KvtAttnLaunch& p, uint64_t w, uint64_t total, uint32_t per_layer,
+                                           uint32_t& layer, uint32_t& kv, uint32_t& tile) {
+  uint32_t rem;
+  if ((total >> 32) == 0u) {   // a 32-bit division costs a fraction of a 64-bit one
+    layer = (uint32_t)w / per_layer;
+    rem = (uint32_t)w - layer * per_layer;
+  } else {
+    layer = (uint32_t)(w / per_layer);
+    rem = (uint32_t)(w - (uint64_t)layer * per_layer);
+  }
+  kv = rem / p.total_tiles;
+  tile = rem - kv * p.total_tiles;
+}
+
+// What is left to do of a tile once it has been decoded: ntok token slots to copy, then nzero to zero on the destination.
+struct TileMove {
+  uint32_t sblk, dblk, s_slot, d_slot, ntok, nzero, layer, kv;
+};
+// The move that lane j holds, in every lane of the warp.
+__device__ __forceinline__ TileMove move_of_lane(const TileMove& mine, int j) {
+  TileMove m;
+  m.sblk = __shfl_sync(0xffffffffu, mine.sblk, j);
+  m.dblk = __shfl_sync(0xffffffffu, mine.dblk, j);
+  m.s_slot = __shfl_sync(0xffffffffu, mine.s_slot, j);
+  m.d_slot = __shfl_sync(0xffffffffu, mine.d_slot, j);
+  m.ntok = __shfl_sync(0xffffffffu, mine.ntok, j);
+  m.nzero = __shfl_sync(0xffffffffu, mine.nzero, j);
+  m.layer = __shfl_sync(0xffffffffu, mine.layer, j);
+  m.kv = __shfl_sync(0xffffffffu, mine.kv, j);
+  return m;
+}
+
 // ---- PTX wrappers -----------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* ptr) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(ptr));
@@ -205,6 +238,34 @@ __device__ __forceinline__ void st_16(void* p, int4 v) {
                : "memory");
 }
 
+__device__ __forceinline__ uint32_t ld_nc_u8(const void* p) {   // volatile: issued here, beside the row's other loads
+  uint32_t v;
+  asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+// 32 bytes per thread in one access where the address allows it (sm_100 has 256-bit loads and stores), else two of 16.
+__device__ __forceinline__ void ld_nc_32(const void* p, bool aligned32, uint32_t w[8]) {
+  if (aligned32) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "l"(p));
+  } else {
+    const int4 a = ld_nc_16(p), b = ld_nc_16(static_cast<const char*>(p) + 16);
+    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+    w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+  }
+}
+__device__ __forceinline__ void st_32(void* p, bool aligned32, const uint32_t w[8]) {
+  if (aligned32) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  } else {
+    st_16(p, make_int4(w[0], w[1], w[2], w[3]));
+    st_16(static_cast<char*>(p) + 16, make_int4(w[4], w[5], w[6], w[7]));
+  }
+}
+
 // ---- block-scaled fp8 helpers -----------------------------------------------------------
 // Scale of a 32-value group: the smallest power of two s with amax / s <= 448 (e4m3 max), stored
 // as a biased UE8M0 exponent byte.  amax == 0 maps to exponent 127 (scale 1).
@@ -227,6 +288,15 @@ __device__ __forceinline__ float scale_from_ue8m0(uint32_t e) { return __uint_as
 __device__ __forceinline__ float bf16lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
+// Largest magnitude of 16 bf16 values, in packed arithmetic: |x| and max are exact, and a NaN loses against a number
+// as it does in fmaxf.
+__device__ __forceinline__ float amax_bf16x16(const uint32_t w[8]) {
+  __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
+#pragma unroll
+  for (int k = 1; k < 8; ++k) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[k])));
+  return fmaxf(fmaxf(0.f, __low2float(m)), __high2float(m));
+}
+
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
   const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
   const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
@@ -236,34 +306,57 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float
 // ---- SIMT tile movers ---------------------------------------------------------------------
 // Rows are enumerated in destination order so that consecutive threads write consecutive
 // destination addresses (NVLink and PCIe like long contiguous write runs).
-struct RowIter {
-  uint32_t ntok, nh;
+//
+// Division of chunk numbers of a tile by one divisor: n * ceil(2^32 / d) >> 32 is floor(n / d) as long as n * d < 2^32,
+// so for tiles of at most 2^16 chunks.  m == 0: d is 1, or the tile is larger than that and takes the plain division.
+struct TileDiv {
+  uint32_t d, m;
+  __device__ __forceinline__ TileDiv(uint32_t d_, uint32_t chunks)
+      : d(d_), m(d_ > 1u && chunks <= 65536u ? 0xffffffffu / d_ + 1u : 0u) {}
+  __device__ __forceinline__ uint32_t quot(uint32_t n) const {
+    if (m != 0u) return __umulhi(n, m);
+    return d == 1u ? n : n / d;
+  }
+};
+// The chunks (16 or 32 bytes) of tiles of one launch: divisors that are the same for every full tile are made once.
+struct TileRows {
+  uint32_t cpr;          // chunks per row
   bool token_inner;
-  __device__ __forceinline__ void decode(uint32_t row, uint32_t& t, uint32_t& h) const {
-    if (token_inner) {
-      h = row / ntok;
-      t = row - h * ntok;
-    } else {
-      t = row / nh;
-      h = row - t * nh;
-    }
+  TileDiv row_div, full_div;
+  __device__ __forceinline__ TileRows(const KvtAttnLaunch& p, uint32_t cpr_)
+      : cpr(cpr_), token_inner(p.dst.token_stride < p.dst.head_stride),
+        row_div(cpr_, p.tile_tokens * p.n_heads * cpr_),
+        full_div(token_inner ? p.tile_tokens : p.n_heads, p.tile_tokens * p.n_heads * cpr_) {}
+};
+struct RowIter {
+  const TileRows& r;
+  uint32_t ntok, chunks;
+  TileDiv inner_div;
+  __device__ __forceinline__ RowIter(const KvtAttnLaunch& p, const TileRows& r_, uint32_t ntok_)
+      : r(r_), ntok(ntok_), chunks(ntok_ * p.n_heads * r_.cpr), inner_div(r_.full_div) {
+    if (r.token_inner && ntok_ != p.tile_tokens) inner_div = TileDiv(ntok_, chunks);
+  }
+  // chunk i, counted in destination order -> token, head and chunk of the row
+  __device__ __forceinline__ void decode(uint32_t i, uint32_t& t, uint32_t& h, uint32_t& c) const {
+    const uint32_t row = r.row_div.quot(i);
+    c = i - row * r.cpr;
+    const uint32_t q = inner_div.quot(row);
+    const uint32_t rest = row - q * inner_div.d;
+    t = r.token_inner ? rest : q;
+    h = r.token_inner ? q : rest;
   }
 };
 
-__device__ __forceinline__ void simt_copy_tile(const KvtAttnLaunch& p, const TileInfo& ti, uint32_t kv,
+__device__ __forceinline__ void simt_copy_tile(const KvtAttnLaunch& p, const TileRows& rows, const TileMove& ti,
                                        const char* __restrict__ src, char* __restrict__ dst, uint32_t tid,
                                        uint32_t nthr) {
-  const uint32_t cpr = p.src.head_bytes >> 4;  // 16-byte chunks per row
-  RowIter it;
-  it.ntok = ti.copy_hi - ti.copy_lo;
-  it.nh = p.n_heads;
-  it.token_inner = p.dst.token_stride < p.dst.head_stride;
-  const uint32_t chunks = it.ntok * it.nh * cpr;
-  const int64_t s_base = (int64_t)ti.sblk * p.src.block_stride + (int64_t)kv * p.src.kv_stride +
-                         (int64_t)(ti.s_slot0 + (ti.copy_lo - ti.tok_lo)) * p.src.token_stride +
+  const RowIter it(p, rows, ti.ntok);
+  const uint32_t chunks = it.chunks;
+  const int64_t s_base = (int64_t)ti.sblk * p.src.block_stride + (int64_t)ti.kv * p.src.kv_stride +
+                         (int64_t)ti.s_slot * p.src.token_stride +
                          (int64_t)p.src_head0 * p.src.head_stride;
-  const int64_t d_base = (int64_t)ti.dblk * p.dst.block_stride + (int64_t)kv * p.dst.kv_stride +
-                         (int64_t)(ti.d_slot0 + (ti.copy_lo - ti.tok_lo)) * p.dst.token_stride +
+  const int64_t d_base = (int64_t)ti.dblk * p.dst.block_stride + (int64_t)ti.kv * p.dst.kv_stride +
+                         (int64_t)ti.d_slot * p.dst.token_stride +
                          (int64_t)p.dst_head0 * p.dst.head_stride;
   constexpr int U = 4;
   for (uint32_t base = tid; base < chunks; base += nthr * U) {
@@ -274,10 +367,8 @@ __device__ __forceinline__ void simt_copy_tile(const KvtAttnLaunch& p, const Til
       const uint32_t i = base + u * nthr;
       doff[u] = -1;
       if (i < chunks) {
-        const uint32_t row = i / cpr;
-        const uint32_t c = i - row * cpr;
-        uint32_t t, h;
-        it.decode(row, t, h);
+        uint32_t t, h, c;
+        it.decode(i, t, h, c);
         v[u] = ld_nc_16(src + s_base + (int64_t)t * p.src.token_stride + (int64_t)h * p.src.head_stride + (c << 4));
         doff[u] = d_base + (int64_t)t * p.dst.token_stride + (int64_t)h * p.dst.head_stride + (c << 4);
       }
@@ -295,24 +386,19 @@ __device__ __forceinline__ void simt_copy_tile(const KvtAttnLaunch& p, const Til
 // destination is quantised into shared memory and leaves as one bulk copy per head (payload) plus one
 // per head (scales): the async-copy engine writes NVLink packets of 256 bytes where the warp's own
 // 16-byte stores leave as 128-byte ones (measured 615 GB/s of link for those against 705 for bulk stores).
-__device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const TileInfo& ti, uint32_t kv,
+__device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const TileRows& rows, const TileMove& ti,
                                        const char* __restrict__ src, char* __restrict__ dst, uint32_t tid,
                                        uint32_t nthr, unsigned char* stage) {
-  const uint32_t cpr = p.src.head_bytes >> 5;  // 32-byte source chunks per row (even: head_dim % 32 == 0)
-  RowIter it;
-  it.ntok = ti.copy_hi - ti.copy_lo;
-  it.nh = p.n_heads;
-  it.token_inner = p.dst.token_stride < p.dst.head_stride;
-  const uint32_t chunks = it.ntok * it.nh * cpr;
-  const uint32_t slot_s = ti.s_slot0 + (ti.copy_lo - ti.tok_lo);
-  const uint32_t slot_d = ti.d_slot0 + (ti.copy_lo - ti.tok_lo);
-  const int64_t s_base = (int64_t)ti.sblk * p.src.block_stride + (int64_t)kv * p.src.kv_stride +
-                         (int64_t)slot_s * p.src.token_stride + (int64_t)p.src_head0 * p.src.head_stride;
+  const uint32_t cpr = rows.cpr;  // 32-byte source chunks per row (even: head_dim % 32 == 0)
+  const RowIter it(p, rows, ti.ntok);
+  const uint32_t chunks = it.chunks;
+  const int64_t s_base = (int64_t)ti.sblk * p.src.block_stride + (int64_t)ti.kv * p.src.kv_stride +
+                         (int64_t)ti.s_slot * p.src.token_stride + (int64_t)p.src_head0 * p.src.head_stride;
   const int64_t d_blk = (int64_t)ti.dblk * p.dst.block_stride;
-  const int64_t d_base = d_blk + (int64_t)kv * p.dst.kv_stride + (int64_t)slot_d * p.dst.token_stride +
+  const int64_t d_base = d_blk + (int64_t)ti.kv * p.dst.kv_stride + (int64_t)ti.d_slot * p.dst.token_stride +
                          (int64_t)p.dst_head0 * p.dst.head_stride;
-  const int64_t sc_base = d_blk + p.dst.scale_base + (int64_t)kv * p.dst.scale_kv_stride +
-                          (int64_t)slot_d * p.dst.scale_token_stride +
+  const int64_t sc_base = d_blk + p.dst.scale_base + (int64_t)ti.kv * p.dst.scale_kv_stride +
+                          (int64_t)ti.d_slot * p.dst.scale_token_stride +
                           (int64_t)p.dst_head0 * p.dst.scale_head_stride;
   // rows of a multiple of 128 values, scale rows 4-byte aligned: scales leave as 32-bit words
   const bool wide_scales = (cpr & 7u) == 0u &&
@@ -320,7 +406,9 @@ __device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const Ti
                              (uint64_t)p.dst.block_stride | reinterpret_cast<uintptr_t>(dst)) & 3u) == 0u;
   const uint32_t run_bytes = it.ntok * p.dst.head_bytes;          // one head's rows of the tile, contiguous in HND
   const uint32_t sc_run = it.ntok * (cpr >> 1);
-  const bool staged = stage != nullptr && wide_scales && it.token_inner && nthr == 32u &&
+  const bool wide_rows = ((reinterpret_cast<uint64_t>(src + s_base) | (uint64_t)p.src.token_stride |
+                           (uint64_t)p.src.head_stride) & 31u) == 0u;
+  const bool staged = stage != nullptr && wide_scales && rows.token_inner && nthr == 32u &&
                       p.dst.token_stride == (int64_t)p.dst.head_bytes && p.dst.scale_token_stride == (int64_t)(cpr >> 1) &&
                       chunks * 16u <= kStagePayload && (chunks >> 1) <= kStageScales &&
                       ((run_bytes | sc_run | (uint32_t)p.dst.head_stride | (uint32_t)p.dst.scale_head_stride) & 15u) == 0u &&
@@ -334,7 +422,6 @@ __device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const Ti
   const uint32_t rounds = (chunks + nthr - 1) / nthr;
   for (uint32_t rnd = 0; rnd < rounds; rnd += 2) {
     uint32_t w[2][8];
-    uint32_t t[2] = {0, 0}, h[2] = {0, 0}, c[2] = {0, 0};
     bool active[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -343,28 +430,20 @@ __device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const Ti
 #pragma unroll
       for (int k = 0; k < 8; ++k) w[u][k] = 0;
       if (active[u]) {
-        const uint32_t row = i / cpr;
-        c[u] = i - row * cpr;
-        it.decode(row, t[u], h[u]);
-        const char* sp = src + s_base + (int64_t)t[u] * p.src.token_stride + (int64_t)h[u] * p.src.head_stride + (c[u] << 5);
-        const int4 a = ld_nc_16(sp);
-        const int4 b = ld_nc_16(sp + 16);
-        w[u][0] = a.x; w[u][1] = a.y; w[u][2] = a.z; w[u][3] = a.w;
-        w[u][4] = b.x; w[u][5] = b.y; w[u][6] = b.z; w[u][7] = b.w;
+        uint32_t t, h, c;
+        it.decode(i, t, h, c);
+        ld_nc_32(src + s_base + (int64_t)t * p.src.token_stride + (int64_t)h * p.src.head_stride + (c << 5), wide_rows, w[u]);
       }
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      float amax = 0.f;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        amax = fmaxf(amax, fabsf(bf16lo(w[u][k])));
-        amax = fmaxf(amax, fabsf(bf16hi(w[u][k])));
-      }
+      float amax = amax_bf16x16(w[u]);
       // the partner lane holds the other half of the 32-value group (all lanes take part in the shuffle)
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
       const uint32_t e = ue8m0_from_amax(amax);
       const float inv = __uint_as_float((254u - e) << 23);  // 1 / 2^(e-127)
+      uint32_t t, h, c;   // decoded again: cheaper than registers held across the loads
+      it.decode((rnd + u) * nthr + tid, t, h, c);
       if (active[u]) {
         int4 q;
         q.x = pack_e4m3x4(bf16lo(w[u][0]) * inv, bf16hi(w[u][0]) * inv, bf16lo(w[u][1]) * inv, bf16hi(w[u][1]) * inv);
@@ -375,7 +454,7 @@ __device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const Ti
           // chunk i of the tile in destination order sits at byte 16 i of the buffer: rows of a head are adjacent
           *reinterpret_cast<int4*>(stage + (((rnd + u) * nthr + tid) << 4)) = q;
         } else {
-          st_16(dst + d_base + (int64_t)t[u] * p.dst.token_stride + (int64_t)h[u] * p.dst.head_stride + (c[u] << 4), q);
+          st_16(dst + d_base + (int64_t)t * p.dst.token_stride + (int64_t)h * p.dst.head_stride + (c << 4), q);
         }
       }
       if (wide_scales) {
@@ -392,13 +471,13 @@ __device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const Ti
             // multiple of eight, so the word is 4-byte aligned whatever the row length
             *reinterpret_cast<uint32_t*>(stage + kStagePayload + (((rnd + u) * nthr + tid) >> 1)) = packed;
           } else {
-            *reinterpret_cast<uint32_t*>(dst + sc_base + (int64_t)t[u] * p.dst.scale_token_stride +
-                                         (int64_t)h[u] * p.dst.scale_head_stride + (c[u] >> 1)) = packed;
+            *reinterpret_cast<uint32_t*>(dst + sc_base + (int64_t)t * p.dst.scale_token_stride +
+                                         (int64_t)h * p.dst.scale_head_stride + (c >> 1)) = packed;
           }
         }
-      } else if (active[u] && (c[u] & 1u) == 0u) {
-        dst[sc_base + (int64_t)t[u] * p.dst.scale_token_stride + (int64_t)h[u] * p.dst.scale_head_stride +
-            (c[u] >> 1)] = static_cast<char>(e);
+      } else if (active[u] && (c & 1u) == 0u) {
+        dst[sc_base + (int64_t)t * p.dst.scale_token_stride + (int64_t)h * p.dst.scale_head_stride +
+            (c >> 1)] = static_cast<char>(e);
       }
     }
   }
@@ -406,7 +485,7 @@ __device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const Ti
     __syncwarp();
     fence_proxy_async();          // the buffer was written through the generic proxy, the copies read it through the async one
     if (tid == 0) {
-      for (uint32_t h = 0; h < it.nh; ++h) {
+      for (uint32_t h = 0; h < p.n_heads; ++h) {
         bulk_store_flat(dst + d_base + (int64_t)h * p.dst.head_stride, smem_u32(stage + h * run_bytes), run_bytes);
         bulk_store_flat(dst + sc_base + (int64_t)h * p.dst.scale_head_stride, smem_u32(stage + kStagePayload + h * sc_run),
                         sc_run);
@@ -417,73 +496,74 @@ __device__ __forceinline__ void simt_quant_tile(const KvtAttnLaunch& p, const Ti
   }
 }
 
-// e4m3 rows + UE8M0 scales -> bf16 rows.  One thread expands 16 values (16 B in, 32 B out).
-__device__ __forceinline__ void simt_dequant_tile(const KvtAttnLaunch& p, const TileInfo& ti, uint32_t kv,
+// e4m3 rows + UE8M0 scales -> bf16 rows.  One thread expands 16 values (16 B in, 32 B out), with four chunks and their
+// scale bytes in flight.
+__device__ __forceinline__ void simt_dequant_tile(const KvtAttnLaunch& p, const TileRows& rows, const TileMove& ti,
                                        const char* __restrict__ src, char* __restrict__ dst, uint32_t tid,
                                        uint32_t nthr) {
-  const uint32_t cpr = p.src.head_bytes >> 4;
-  RowIter it;
-  it.ntok = ti.copy_hi - ti.copy_lo;
-  it.nh = p.n_heads;
-  it.token_inner = p.dst.token_stride < p.dst.head_stride;
-  const uint32_t chunks = it.ntok * it.nh * cpr;
-  const uint32_t slot_s = ti.s_slot0 + (ti.copy_lo - ti.tok_lo);
-  const uint32_t slot_d = ti.d_slot0 + (ti.copy_lo - ti.tok_lo);
+  const RowIter it(p, rows, ti.ntok);
+  const uint32_t chunks = it.chunks;
   const int64_t s_blk = (int64_t)ti.sblk * p.src.block_stride;
-  const int64_t s_base = s_blk + (int64_t)kv * p.src.kv_stride + (int64_t)slot_s * p.src.token_stride +
+  const int64_t s_base = s_blk + (int64_t)ti.kv * p.src.kv_stride + (int64_t)ti.s_slot * p.src.token_stride +
                          (int64_t)p.src_head0 * p.src.head_stride;
-  const int64_t sc_base = s_blk + p.src.scale_base + (int64_t)kv * p.src.scale_kv_stride +
-                          (int64_t)slot_s * p.src.scale_token_stride +
+  const int64_t sc_base = s_blk + p.src.scale_base + (int64_t)ti.kv * p.src.scale_kv_stride +
+                          (int64_t)ti.s_slot * p.src.scale_token_stride +
                           (int64_t)p.src_head0 * p.src.scale_head_stride;
-  const int64_t d_base = (int64_t)ti.dblk * p.dst.block_stride + (int64_t)kv * p.dst.kv_stride +
-                         (int64_t)slot_d * p.dst.token_stride + (int64_t)p.dst_head0 * p.dst.head_stride;
-  for (uint32_t i = tid; i < chunks; i += nthr) {
-    const uint32_t row = i / cpr;
-    const uint32_t c = i - row * cpr;
-    uint32_t t, h;
-    it.decode(row, t, h);
-    const int4 q = ld_nc_16(src + s_base + (int64_t)t * p.src.token_stride + (int64_t)h * p.src.head_stride + (c << 4));
-    const uint32_t e = static_cast<uint8_t>(
-        src[sc_base + (int64_t)t * p.src.scale_token_stride + (int64_t)h * p.src.scale_head_stride + (c >> 1)]);
-    const float s = scale_from_ue8m0(e);
-    const uint32_t qw[4] = {(uint32_t)q.x, (uint32_t)q.y, (uint32_t)q.z, (uint32_t)q.w};
-    uint32_t o[8];
+  const int64_t d_base = (int64_t)ti.dblk * p.dst.block_stride + (int64_t)ti.kv * p.dst.kv_stride +
+                         (int64_t)ti.d_slot * p.dst.token_stride + (int64_t)p.dst_head0 * p.dst.head_stride;
+  const bool wide_rows = ((reinterpret_cast<uint64_t>(dst + d_base) | (uint64_t)p.dst.token_stride |
+                           (uint64_t)p.dst.head_stride) & 31u) == 0u;
+  constexpr int U = 4;
+  for (uint32_t base = tid; base < chunks; base += nthr * U) {
+    int4 q[U];
+    uint32_t e[U];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(qw[k] & 0xffffu), __NV_E4M3);
-      const __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(qw[k] >> 16), __NV_E4M3);
-      const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&h01));
-      const float2 f23 = __half22float2(*reinterpret_cast<const __half2*>(&h23));
-      const __nv_bfloat162 b01 = __floats2bfloat162_rn(f01.x * s, f01.y * s);
-      const __nv_bfloat162 b23 = __floats2bfloat162_rn(f23.x * s, f23.y * s);
-      o[2 * k] = *reinterpret_cast<const uint32_t*>(&b01);
-      o[2 * k + 1] = *reinterpret_cast<const uint32_t*>(&b23);
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + u * nthr;
+      if (i < chunks) {
+        uint32_t t, h, c;
+        it.decode(i, t, h, c);
+        q[u] = ld_nc_16(src + s_base + (int64_t)t * p.src.token_stride + (int64_t)h * p.src.head_stride + (c << 4));
+        e[u] = ld_nc_u8(src + sc_base + (int64_t)t * p.src.scale_token_stride + (int64_t)h * p.src.scale_head_stride + (c >> 1));
+      }
     }
-    char* dp = dst + d_base + (int64_t)t * p.dst.token_stride + (int64_t)h * p.dst.head_stride + (c << 5);
-    st_16(dp, make_int4(o[0], o[1], o[2], o[3]));
-    st_16(dp + 16, make_int4(o[4], o[5], o[6], o[7]));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + u * nthr;
+      if (i >= chunks) break;
+      const float s = scale_from_ue8m0(e[u]);
+      const uint32_t qw[4] = {(uint32_t)q[u].x, (uint32_t)q[u].y, (uint32_t)q[u].z, (uint32_t)q[u].w};
+      uint32_t o[8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const __half2_raw h01 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(qw[k] & 0xffffu), __NV_E4M3);
+        const __half2_raw h23 = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(qw[k] >> 16), __NV_E4M3);
+        const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&h01));
+        const float2 f23 = __half22float2(*reinterpret_cast<const __half2*>(&h23));
+        const __nv_bfloat162 b01 = __floats2bfloat162_rn(f01.x * s, f01.y * s);
+        const __nv_bfloat162 b23 = __floats2bfloat162_rn(f23.x * s, f23.y * s);
+        o[2 * k] = *reinterpret_cast<const uint32_t*>(&b01);
+        o[2 * k + 1] = *reinterpret_cast<const uint32_t*>(&b23);
+      }
+      uint32_t t, h, c;   // decoded again: cheaper than registers held across the loads
+      it.decode(i, t, h, c);
+      st_32(dst + d_base + (int64_t)t * p.dst.token_stride + (int64_t)h * p.dst.head_stride + (c << 5), wide_rows, o);
+    }
   }
 }
 
 // Zero destination slots [copy_hi, zero_hi) of a tile (tail pad of the last block).
-__device__ __forceinline__ void simt_zero_tail(const KvtAttnLaunch& p, const TileInfo& ti, uint32_t kv,
+__device__ __forceinline__ void simt_zero_tail(const KvtAttnLaunch& p, const TileMove& ti,
                                                char* __restrict__ dst, uint32_t tid, uint32_t nthr) {
-  const uint32_t ntok = ti.zero_hi - ti.copy_hi;
-  if (ntok == 0) return;
-  const uint32_t cpr = p.dst.head_bytes >> 4;
-  RowIter it;
-  it.ntok = ntok;
-  it.nh = p.n_heads;
-  it.token_inner = p.dst.token_stride < p.dst.head_stride;
-  const uint32_t chunks = ntok * it.nh * cpr;
-  const int64_t d_base = (int64_t)ti.dblk * p.dst.block_stride + (int64_t)kv * p.dst.kv_stride +
-                         (int64_t)(ti.d_slot0 + (ti.copy_hi - ti.tok_lo)) * p.dst.token_stride +
+  const TileRows rows(p, p.dst.head_bytes >> 4);
+  const RowIter it(p, rows, ti.nzero);
+  const uint32_t chunks = it.chunks;
+  const int64_t d_base = (int64_t)ti.dblk * p.dst.block_stride + (int64_t)ti.kv * p.dst.kv_stride +
+                         (int64_t)(ti.d_slot + ti.ntok) * p.dst.token_stride +
                          (int64_t)p.dst_head0 * p.dst.head_stride;
   for (uint32_t i = tid; i < chunks; i += nthr) {
-    const uint32_t row = i / cpr;
-    const uint32_t c = i - row * cpr;
-    uint32_t t, h;
-    it.decode(row, t, h);
+    uint32_t t, h, c;
+    it.decode(i, t, h, c);
     st_16(dst + d_base + (int64_t)t * p.dst.token_stride + (int64_t)h * p.dst.head_stride + (c << 4),
           make_int4(0, 0, 0, 0));
   }
@@ -508,28 +588,47 @@ __device__ __forceinline__ void simt_pass(const KvtAttnLaunch& p, uint64_t total
   if (me >= owners) return;   // a block size that is not a multiple of the group: the odd warps sit out
   unsigned char* stage = (GROUP == 1 && MODE == KVT_MODE_BF16_TO_MXFP8 && stage_base != nullptr)
                              ? stage_base + (size_t)me * kStagePerWarp : nullptr;
-  for (uint64_t w = (uint64_t)blockIdx.x * owners + me; w < total; w += (uint64_t)gridDim.x * owners) {
-    const uint32_t layer = (uint32_t)(w / per_layer);
-    const uint32_t rem = (uint32_t)(w - (uint64_t)layer * per_layer);
-    const uint32_t kv = rem / p.total_tiles;
-    const uint32_t tile = rem - kv * p.total_tiles;
-    const TileInfo ti = decode_tile(p, tile);
-    if (!ti.ok) {
-      if (tid == 0) set_status(p.status, KVT_ERR_BLOCK_RANGE, tile);
-      continue;
-    }
-    const char* src = reinterpret_cast<const char*>(p.src_layers[p.layer_begin + layer]);
-    char* dst = reinterpret_cast<char*>(p.dst_layers[p.layer_begin + layer]);
-    if (ti.copy_hi > ti.copy_lo) {
-      if constexpr (MODE == KVT_MODE_COPY) {
-        if (!(USE_TMA && tile_is_full(p, ti))) simt_copy_tile(p, ti, kv, src, dst, tid, nthr);
-      } else if constexpr (MODE == KVT_MODE_BF16_TO_MXFP8) {
-        simt_quant_tile(p, ti, kv, src, dst, tid, nthr, stage);
+  const TileRows rows(p, MODE == KVT_MODE_BF16_TO_MXFP8 ? p.src.head_bytes >> 5 : p.src.head_bytes >> 4);
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t step = (uint64_t)gridDim.x * owners;
+  // The walk from a tile number to its block ids is a chain of dependent loads: the lanes walk the owner's next 32 tiles
+  // at once, then the tiles are moved one after the other.
+  for (uint64_t first = (uint64_t)blockIdx.x * owners + me; first < total; first += 32u * step) {
+    const uint64_t w = first + lane * step;
+    TileMove mine = {};
+    bool work = false;
+    if (w < total) {
+      uint32_t tile;
+      split_work(p, w, total, per_layer, mine.layer, mine.kv, tile);
+      const TileInfo ti = decode_tile(p, tile);
+      if (!ti.ok) {
+        if (tid < 32u) set_status(p.status, KVT_ERR_BLOCK_RANGE, tile);
       } else {
-        simt_dequant_tile(p, ti, kv, src, dst, tid, nthr);
+        mine.sblk = ti.sblk;
+        mine.dblk = ti.dblk;
+        mine.s_slot = ti.s_slot0 + (ti.copy_lo - ti.tok_lo);
+        mine.d_slot = ti.d_slot0 + (ti.copy_lo - ti.tok_lo);
+        mine.ntok = ti.copy_hi - ti.copy_lo;
+        mine.nzero = ti.zero_hi - ti.copy_hi;
+        // full tiles (nothing to zero) went through the TMA pass
+        work = (mine.ntok | mine.nzero) != 0u && !(MODE == KVT_MODE_COPY && USE_TMA && tile_is_full(p, ti));
       }
     }
-    if (ti.zero_hi > ti.copy_hi) simt_zero_tail(p, ti, kv, dst, tid, nthr);
+    for (unsigned todo = __ballot_sync(0xffffffffu, work); todo != 0u; todo &= todo - 1u) {
+      const TileMove ti = move_of_lane(mine, __ffs(todo) - 1);
+      const char* src = reinterpret_cast<const char*>(p.src_layers[p.layer_begin + ti.layer]);
+      char* dst = reinterpret_cast<char*>(p.dst_layers[p.layer_begin + ti.layer]);
+      if (ti.ntok != 0u) {
+        if constexpr (MODE == KVT_MODE_COPY) {
+          simt_copy_tile(p, rows, ti, src, dst, tid, nthr);
+        } else if constexpr (MODE == KVT_MODE_BF16_TO_MXFP8) {
+          simt_quant_tile(p, rows, ti, src, dst, tid, nthr, stage);
+        } else {
+          simt_dequant_tile(p, rows, ti, src, dst, tid, nthr);
+        }
+      }
+      if (ti.nzero != 0u) simt_zero_tail(p, ti, dst, tid, nthr);
+    }
   }
   if (stage != nullptr) {
     // the bulk stores of the last tile must be complete before this CTA reports the launch done
@@ -606,10 +705,9 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
         ti.sblk = ti.dblk = ti.s_slot0 = ti.d_slot0 = 0;
         uint32_t layer = 0, kv = 0;
         if (w < total) {
-          layer = (uint32_t)(w / per_layer);
-          const uint32_t rem = (uint32_t)(w - (uint64_t)layer * per_layer);
-          kv = rem / p.total_tiles;
-          ti = decode_tile(p, rem - kv * p.total_tiles);
+          uint32_t tile;
+          split_work(p, w, total, per_layer, layer, kv, tile);
+          ti = decode_tile(p, tile);
           full = ti.ok && tile_is_full(p, ti);  // bad tiles are reported by the SIMT pass
         }
         const unsigned any = __ballot_sync(0xffffffffu, w < total);
