@@ -11,13 +11,13 @@
 // memory.  No staging buffer and no library copy is involved.
 //
 // Work unit ("tile"): tile_tokens consecutive token slots of one request for one of K / V in
-// one layer, all transferred heads.  Full tiles move with TMA: one elected thread issues a
+// one layer, all transferred heads.  Copies move with TMA: one elected thread issues a
 // cp.async.bulk.tensor load of the {head_bytes, heads, tokens} box into shared memory and a
 // cp.async.bulk.tensor store of the same box through a destination map whose strides encode
 // the destination layout, so the NHD<->HND permutation is done by the copy engine and the SM
-// issues two instructions per 8-32 KiB.  Ragged edges (a chunk that starts or ends inside a
-// block), the fp8 paths and layouts TMA cannot describe run on a 16-byte-vector SIMT path in
-// the same launch.  TMA loads never use cluster multicast.
+// issues two instructions per 8-32 KiB.  A ragged edge (a chunk that starts or ends inside a
+// block) is loaded as a whole tile and leaves as one untiled bulk store per contiguous run of
+// its own slots.  The fp8 paths and layouts TMA cannot describe run on a vector SIMT path.  TMA loads never use cluster multicast.
 //
 // Every wait is bounded; on a bad block id or a timeout the kernel records a status word and
 // skips the access instead of faulting.
@@ -110,10 +110,6 @@ __device__ __forceinline__ TileInfo decode_tile(const KvtAttnLaunch& p, uint32_t
     if (ti.dblk >= p.dst.num_blocks) ti.ok = false;
   }
   return ti;
-}
-
-__device__ __forceinline__ bool tile_is_full(const KvtAttnLaunch& p, const TileInfo& ti) {
-  return ti.copy_lo == ti.tok_lo && ti.copy_hi == ti.tok_lo + p.tile_tokens;
 }
 
 // Work item w of a launch -> layer, K or V, tile of the layer.
@@ -217,6 +213,9 @@ __device__ __forceinline__ void bulk_store_flat_hint(void* gdst, uint32_t smem_s
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(gdst),
                "r"(smem_src), "r"(bytes), "l"(pol)
                : "memory");
+}
+__device__ __forceinline__ void bulk_store_run(char* gdst, uint32_t smem_src, uint32_t bytes, bool hinted, uint64_t pol) {
+  if (hinted) bulk_store_flat_hint(gdst, smem_src, bytes, pol); else bulk_store_flat(gdst, smem_src, bytes);
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N>
@@ -610,15 +609,14 @@ __device__ __forceinline__ void simt_pass(const KvtAttnLaunch& p, uint64_t total
         mine.d_slot = ti.d_slot0 + (ti.copy_lo - ti.tok_lo);
         mine.ntok = ti.copy_hi - ti.copy_lo;
         mine.nzero = ti.zero_hi - ti.copy_hi;
-        // full tiles (nothing to zero) went through the TMA pass
-        work = (mine.ntok | mine.nzero) != 0u && !(MODE == KVT_MODE_COPY && USE_TMA && tile_is_full(p, ti));
+        work = (USE_TMA ? mine.nzero : mine.ntok | mine.nzero) != 0u;   // the TMA pass copies
       }
     }
     for (unsigned todo = __ballot_sync(0xffffffffu, work); todo != 0u; todo &= todo - 1u) {
       const TileMove ti = move_of_lane(mine, __ffs(todo) - 1);
       const char* src = reinterpret_cast<const char*>(p.src_layers[p.layer_begin + ti.layer]);
       char* dst = reinterpret_cast<char*>(p.dst_layers[p.layer_begin + ti.layer]);
-      if (ti.ntok != 0u) {
+      if (ti.ntok != 0u && !USE_TMA) {
         if constexpr (MODE == KVT_MODE_COPY) {
           simt_copy_tile(p, rows, ti, src, dst, tid, nthr);
         } else if constexpr (MODE == KVT_MODE_BF16_TO_MXFP8) {
@@ -636,6 +634,31 @@ __device__ __forceinline__ void simt_pass(const KvtAttnLaunch& p, uint64_t total
     __syncwarp();
     fence_proxy_async();
   }
+}
+
+// Token slots [lo, lo + n) of a tile in shared memory leave as untiled bulk stores, one per run that both sides hold
+// contiguously: per head for an HND page, per token (or one in all) for an NHD page.  `dst` is the address of slot lo,
+// first moved head.
+__device__ __forceinline__ void bulk_store_slots(const KvtAttnLaunch& p, char* dst, uint32_t tile_smem, uint32_t lo, uint32_t n,
+                                                 bool hinted, uint64_t pol) {
+  const bool token_inner = p.tile_order != 0u;
+  const uint32_t hb = p.dst.head_bytes;
+  const uint32_t s_outer = (token_inner ? p.tile_tokens : p.n_heads) * hb;
+  const int64_t d_outer = token_inner ? p.dst.head_stride : p.dst.token_stride;
+  const int64_t d_inner = token_inner ? p.dst.token_stride : p.dst.head_stride;
+  uint32_t n_outer = token_inner ? p.n_heads : n, n_inner = token_inner ? n : p.n_heads, run = hb;
+  if (d_inner == (int64_t)hb) {
+    run = n_inner * hb;
+    n_inner = 1;
+    if (s_outer == run && d_outer == (int64_t)run) {
+      run *= n_outer;
+      n_outer = 1;
+    }
+  }
+  const uint32_t sm = tile_smem + lo * (token_inner ? hb : s_outer);
+  for (uint32_t o = 0; o < n_outer; ++o)
+    for (uint32_t i = 0; i < n_inner; ++i)
+      bulk_store_run(dst + (int64_t)o * d_outer + (int64_t)i * d_inner, sm + o * s_outer + i * hb, run, hinted, pol);
 }
 
 // ---- the kernel ---------------------------------------------------------------------------
@@ -662,8 +685,10 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
       // of dependent loads, so doing it on one thread would serialise ~1 us per tile); lane 0
       // runs the software pipeline: at most n_stages-1 loads in flight, one store behind.
       const uint32_t lane = threadIdx.x;
-      // dmap == nullptr: the tile is one contiguous run of the destination, stored by an untiled bulk copy to `flat`
-      struct Slot { const void* dmap; char* flat; int c1, c2, c3, c4; };
+      // dmap == nullptr: the tile (or the n slots from lo that the request has in it) is stored by untiled bulk copies
+      // from `flat` on.  A partly filled tile is LOADED whole: its other slots are cache memory of the same block, read
+      // and dropped.
+      struct Slot { const void* dmap; char* flat; int c1, c2, c3, c4; uint32_t lo, n; };
       Slot slots[kMaxStages];
       uint32_t issued = 0, stored = 0;
       bool failed = false;
@@ -687,9 +712,10 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
           return;
         }
         const uint32_t sm = smem_u32(smem + (size_t)s * tile_bytes);
-        if (slots[s].dmap == nullptr) {
-          if (hinted) bulk_store_flat_hint(slots[s].flat, sm, tile_bytes, pol);
-          else bulk_store_flat(slots[s].flat, sm, tile_bytes);
+        if (slots[s].n != p.tile_tokens) {
+          bulk_store_slots(p, slots[s].flat, sm, slots[s].lo, slots[s].n, hinted, pol);
+        } else if (slots[s].dmap == nullptr) {
+          bulk_store_run(slots[s].flat, sm, tile_bytes, hinted, pol);
         } else if (hinted) {
           tma_store_5d_hint(slots[s].dmap, sm, 0, slots[s].c1, slots[s].c2, slots[s].c3, slots[s].c4, pol);
         } else {
@@ -700,28 +726,30 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
       };
       for (uint64_t batch = 0;; batch += 32) {
         const uint64_t w = blockIdx.x + (batch + lane) * (uint64_t)gridDim.x;
-        bool full = false;
+        bool mine = false;
         TileInfo ti;
-        ti.sblk = ti.dblk = ti.s_slot0 = ti.d_slot0 = 0;
+        ti.sblk = ti.dblk = ti.s_slot0 = ti.d_slot0 = ti.tok_lo = ti.copy_lo = ti.copy_hi = 0;
         uint32_t layer = 0, kv = 0;
         if (w < total) {
           uint32_t tile;
           split_work(p, w, total, per_layer, layer, kv, tile);
           ti = decode_tile(p, tile);
-          full = ti.ok && tile_is_full(p, ti);  // bad tiles are reported by the SIMT pass
+          mine = ti.ok && ti.copy_hi > ti.copy_lo;  // bad tiles are reported by the SIMT pass
         }
         const unsigned any = __ballot_sync(0xffffffffu, w < total);
-        unsigned fullmask = __ballot_sync(0xffffffffu, full);
+        unsigned todo = __ballot_sync(0xffffffffu, mine);
         if (any == 0u) break;
-        while (fullmask != 0u) {
-          const int j = __ffs(fullmask) - 1;
-          fullmask &= fullmask - 1u;
+        while (todo != 0u) {
+          const int j = __ffs(todo) - 1;
+          todo &= todo - 1u;
           const uint32_t j_sblk = __shfl_sync(0xffffffffu, ti.sblk, j);
           const uint32_t j_dblk = __shfl_sync(0xffffffffu, ti.dblk, j);
           const uint32_t j_ss = __shfl_sync(0xffffffffu, ti.s_slot0, j);
           const uint32_t j_ds = __shfl_sync(0xffffffffu, ti.d_slot0, j);
           const uint32_t j_layer = __shfl_sync(0xffffffffu, layer, j);
           const uint32_t j_kv = __shfl_sync(0xffffffffu, kv, j);
+          const uint32_t j_lo = __shfl_sync(0xffffffffu, ti.copy_lo - ti.tok_lo, j);
+          const uint32_t j_n = __shfl_sync(0xffffffffu, ti.copy_hi - ti.copy_lo, j);
           if (lane == 0 && !failed) {
             if (n_stages == 1) {
               if (issued > stored) consume_one();
@@ -749,11 +777,13 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
               slots[s].dmap = flat_store ? nullptr : dmap;
               slots[s].flat = reinterpret_cast<char*>(p.dst_layers[p.layer_begin + j_layer]) +
                               (int64_t)j_dblk * p.dst.block_stride + (int64_t)j_kv * p.dst.kv_stride +
-                              (int64_t)j_ds * p.dst.token_stride + (int64_t)p.dst_head0 * p.dst.head_stride;
+                              (int64_t)(j_ds + j_lo) * p.dst.token_stride + (int64_t)p.dst_head0 * p.dst.head_stride;
               slots[s].c1 = token_inner ? (int)j_ds : (int)p.dst_head0;
               slots[s].c2 = token_inner ? (int)p.dst_head0 : (int)j_ds;
               slots[s].c3 = (int)j_dblk;
               slots[s].c4 = (int)j_kv;
+              slots[s].lo = j_lo;
+              slots[s].n = j_n;
               ++issued;
             }
           }
@@ -768,7 +798,7 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
     }
   }
 
-  // SIMT pass: everything the TMA pass does not take.
+  // SIMT pass: everything the TMA pass does not take (with TMA: tail zeros and the report of bad tiles).
   // without TMA tiles a non-zero tile_bytes says that every warp owns a staging buffer of that size
   unsigned char* stage_base = (!USE_TMA && tile_bytes == kStagePerWarp) ? smem : nullptr;
   if (warp_tiles == 1u) {
