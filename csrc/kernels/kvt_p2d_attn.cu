@@ -21,6 +21,7 @@
 //
 // Every wait is bounded; on a bad block id or a timeout the kernel records a status word and
 // skips the access instead of faulting.
+#include <algorithm>
 #include <atomic>
 
 #include <cuda.h>
@@ -992,16 +993,29 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
   // than one deep software pipeline per SM, and they let launches on different streams share SMs.
   int grid = grid_ctas > 0 ? grid_ctas : 4 * sms;
   const uint64_t total = (uint64_t)(a.layer_end - a.layer_begin) * a.total_tiles * a.src.kv_count;
+  const bool tma = use_tma && a.mode == KVT_MODE_COPY && a.src_maps != nullptr && a.dst_maps != nullptr;
+  const uint32_t tile_bytes = tma ? a.src.head_bytes * a.n_heads * a.tile_tokens : 0u;
+  int resident = grid;   // CTAs that are on the GPU together
+  if (tma && grid_ctas <= 0 && a.dst_remote == 0 && tile_bytes != 0) {
+    // A long launch inside one GPU: CTAs of 128 KiB of tiles, handed to the SMs as they become free, six at a time on
+    // each.  With a fixed share for each of four CTAs per SM the slowest one ends the launch: 32 layers of 8192 tokens
+    // and 8 heads (1 GiB) took 361 us so and 341 with 3 to 4 tiles a CTA (343 with 7, 349 with 14); at 4 heads and
+    // 191 tiles a layer 77 us both ways, and 83 with one tile a CTA.  Over NVLink the link bounds either.
+    const uint64_t tiles = tile_bytes < (128u << 10) ? (128u << 10) / tile_bytes : 1u;
+    const uint64_t want = (total + tiles - 1) / tiles;
+    if (want > (uint64_t)grid) {
+      grid = (int)(want < (1u << 30) ? want : (1u << 30));
+      resident = grid < 6 * sms ? grid : 6 * sms;
+    }
+  }
   if ((uint64_t)grid > total) grid = (int)total;
   if (threads <= 0) threads = use_tma ? 128 : 512;
   if (threads > 512) threads = 512;
   threads = (threads + 31) / 32 * 32;
-  const bool tma = use_tma && a.mode == KVT_MODE_COPY && a.src_maps != nullptr && a.dst_maps != nullptr;
   if (tma) {
-    const uint32_t tile_bytes = a.src.head_bytes * a.n_heads * a.tile_tokens;
     if (tile_bytes % 128 != 0 || tile_bytes > kSmemBudget) return (int)cudaErrorInvalidValue;
     // the shared-memory budget of an SM is split among the CTAs meant to live on it together
-    const uint32_t ctas_per_sm = sms > 0 ? (uint32_t)((grid + sms - 1) / sms) : 1u;
+    const uint32_t ctas_per_sm = sms > 0 ? (uint32_t)((std::min(grid, resident) + sms - 1) / sms) : 1u;
     uint32_t stages = kSmemBudget / (ctas_per_sm > 0 ? ctas_per_sm : 1u) / tile_bytes;
     if (stages > (uint32_t)kMaxStages) stages = kMaxStages;
     if (stages < 1) stages = 1;

@@ -263,7 +263,7 @@ void BatchEngine::launch_attn(const DeviceAttnParams& params, const PackedPlan& 
   a.dst_remote = cfg_.dst_remote ? 1u : 0u;
   a.tile_order = tile_order_;
   a.store_form = store_form_;
-  cuda_check(kvt_launch_p2d_attn(&a, grid(), 0, use_tma_ ? 1 : 0, st.stream()), "kvt_launch_p2d_attn");
+  cuda_check(kvt_launch_p2d_attn(&a, cfg_.one_gpu && cfg_.grid_ctas <= 0 && env_kernel_copy_sm_usage() >= 1.0 ? 0 : grid(), 0, use_tma_ ? 1 : 0, st.stream()), "kvt_launch_p2d_attn");
 }
 
 void BatchEngine::ensure_walk_arrays() {

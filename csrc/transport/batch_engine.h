@@ -37,6 +37,7 @@ struct BatchEngineConfig {
   size_t plan_capacity = 2u << 20;   // bytes per slot
   bool stamps = false;               // GPU timer stamps around every batch (DeviceUs in the metrics)
   bool dst_remote = false;           // the destination is another GPU's memory (quantiser staging, see kvt_kernels.h)
+  bool one_gpu = false;              // both caches live on this GPU: launches take the kernel's own grid rule
   int grid_ctas = 0;                 // 0: four CTAs per SM scaled by the SM-usage knob
 };
 
