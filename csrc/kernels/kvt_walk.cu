@@ -145,28 +145,58 @@ __device__ __forceinline__ bool bulk_ok(const Resolved& r) {
          ((reinterpret_cast<uintptr_t>(r.src) | reinterpret_cast<uintptr_t>(r.dst) | r.len) & 15u) == 0;
 }
 
-// One warp copies (or zero-fills) the n pieces of a unit.
+// What lane j resolved, in every lane of the warp.
+__device__ __forceinline__ Resolved resolved_of_lane(const Resolved& mine, int j) {
+  Resolved r;
+  r.src = reinterpret_cast<const char*>(__shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(mine.src), j));
+  r.dst = reinterpret_cast<char*>(__shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(mine.dst), j));
+  r.src_step = __shfl_sync(0xffffffffu, mine.src_step, j);
+  r.dst_step = __shfl_sync(0xffffffffu, mine.dst_step, j);
+  r.len = __shfl_sync(0xffffffffu, mine.len, j);
+  r.n = __shfl_sync(0xffffffffu, mine.n, j);
+  r.zero = __shfl_sync(0xffffffffu, (uint32_t)mine.zero, j) != 0u;
+  return r;
+}
+
+// The n pieces of a unit in words of V: U loads of a lane are in flight before the first of their stores.
+template <typename V, int U>
+__device__ __forceinline__ void warp_words(const Resolved& r, uint32_t lane) {
+  const uint32_t cpp = r.len / (uint32_t)sizeof(V);
+  const uint32_t total = cpp * r.n;
+  // i / cpp by multiplication with ceil(2^32 / cpp): exact while i * cpp < 2^32, so for units of up to 2^16 words.
+  // m == 0: one piece, pieces of one word, or a larger unit (divided).
+  const uint32_t m = r.n > 1u && cpp > 1u && total <= 65536u ? 0xffffffffu / cpp + 1u : 0u;
+  auto piece_of = [&](uint32_t i) { return m != 0u ? __umulhi(i, m) : (r.n == 1u ? 0u : i / cpp); };
+  for (uint32_t base = lane; base < total; base += 32u * U) {
+    V v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + 32u * u;
+      v[u] = V{};
+      if (i < total && !r.zero) {
+        const uint32_t j = piece_of(i);
+        v[u] = *reinterpret_cast<const V*>(r.src + (int64_t)j * r.src_step + (uint64_t)(i - j * cpp) * sizeof(V));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = base + 32u * u;
+      if (i < total) {
+        const uint32_t j = piece_of(i);
+        *reinterpret_cast<V*>(r.dst + (int64_t)j * r.dst_step + (uint64_t)(i - j * cpp) * sizeof(V)) = v[u];
+      }
+    }
+  }
+}
+
+// One warp copies (or zero-fills) the n pieces of a unit, in the widest words that both sides allow.
 __device__ __forceinline__ void warp_pieces(const Resolved& r, uint32_t lane) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(r.src) | reinterpret_cast<uintptr_t>(r.dst) | (uintptr_t)r.src_step |
                       (uintptr_t)r.dst_step | r.len;
   if ((a & 15u) == 0) {
-    const uint32_t cpp = r.len >> 4;                 // 16-byte chunks per piece
-    const uint32_t total = cpp * r.n;
-    for (uint32_t i = lane; i < total; i += 32) {
-      const uint32_t j = i / cpp, c = i - j * cpp;
-      int4 v = make_int4(0, 0, 0, 0);
-      if (!r.zero) v = *reinterpret_cast<const int4*>(r.src + (int64_t)j * r.src_step + ((int64_t)c << 4));
-      *reinterpret_cast<int4*>(r.dst + (int64_t)j * r.dst_step + ((int64_t)c << 4)) = v;
-    }
+    warp_words<int4, 4>(r, lane);
   } else if ((a & 3u) == 0) {
-    const uint32_t cpp = r.len >> 2;
-    const uint32_t total = cpp * r.n;
-    for (uint32_t i = lane; i < total; i += 32) {
-      const uint32_t j = i / cpp, c = i - j * cpp;
-      int v = 0;
-      if (!r.zero) v = *reinterpret_cast<const int*>(r.src + (int64_t)j * r.src_step + ((int64_t)c << 2));
-      *reinterpret_cast<int*>(r.dst + (int64_t)j * r.dst_step + ((int64_t)c << 2)) = v;
-    }
+    warp_words<int, 4>(r, lane);
   } else {
     const uint64_t total = (uint64_t)r.len * r.n;
     for (uint64_t i = lane; i < total; i += 32) {
@@ -176,7 +206,42 @@ __device__ __forceinline__ void warp_pieces(const Resolved& r, uint32_t lane) {
   }
 }
 
-__global__ void __launch_bounds__(256) kvt_walk_kernel(const __grid_constant__ KvtWalkLaunch p, const uint32_t n_stages) {
+// The SIMT warps' share, warp w0 of nw in this CTA: the SIMT class, then the units of the bulk class whose addresses do
+// not allow the TMA engine to take them.  Lanes resolve 32 units at once (a unit's block tables are a chain of dependent
+// loads), then the warp moves those that are its to move one after the other.
+__device__ __forceinline__ void simt_units(const KvtWalkLaunch& p, uint32_t w0, uint32_t nw, uint32_t lane) {
+  const uint32_t n_layers = p.layer_end - p.layer_begin;
+#pragma unroll 1
+  for (int leftovers = 0; leftovers < 2; ++leftovers) {
+    const uint64_t units = leftovers ? p.bulk_units : p.simt_units;
+    const uint64_t total = units * n_layers;
+    const KvtWalkOp* ops = leftovers ? p.ops : p.ops + p.n_bulk_ops;
+    const uint32_t n_ops = leftovers ? p.n_bulk_ops : p.n_simt_ops;
+#pragma unroll 1
+    for (uint64_t k = w0;; k += 32ull * nw) {
+      const uint64_t first = blockIdx.x + k * (uint64_t)gridDim.x;
+      if (first >= total) break;
+      const uint64_t w = first + (uint64_t)(lane * nw) * gridDim.x;
+      Resolved mine;
+      mine.src = nullptr;
+      mine.dst = nullptr;
+      mine.src_step = mine.dst_step = 0;
+      mine.len = mine.n = 0;
+      mine.zero = false;
+      if (w < total) {
+        uint64_t unit;
+        uint32_t layer;
+        split_unit(w, units, &unit, &layer);
+        // the bulk pass reports the errors of its own units
+        mine = resolve(p, ops, n_ops, unit, p.layer_begin + layer, leftovers == 0);
+      }
+      for (unsigned todo = __ballot_sync(0xffffffffu, mine.n != 0 && !(leftovers && bulk_ok(mine))); todo != 0u; todo &= todo - 1u)
+        warp_pieces(resolved_of_lane(mine, __ffs(todo) - 1), lane);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256, 4) kvt_walk_kernel(const __grid_constant__ KvtWalkLaunch p, const uint32_t n_stages) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)n_stages * KVT_WALK_SEG);
   if (threadIdx.x == 0) {
@@ -188,8 +253,7 @@ __global__ void __launch_bounds__(256) kvt_walk_kernel(const __grid_constant__ K
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t n_layers = p.layer_end - p.layer_begin;
   const KvtWalkOp* bulk_ops = p.ops;
-  const KvtWalkOp* simt_ops = p.ops + p.n_bulk_ops;
-  const uint64_t bulk_total = p.bulk_units * n_layers, simt_total = p.simt_units * n_layers;
+  const uint64_t bulk_total = p.bulk_units * n_layers;
   if (warp == 0) {
     // ---- bulk pass: lanes decode 32 units at a time, lane 0 runs the pipeline -----------------------
     char* sdst[kMaxStagesW] = {};
@@ -268,25 +332,7 @@ __global__ void __launch_bounds__(256) kvt_walk_kernel(const __grid_constant__ K
   } else {
     // ---- SIMT pass: the ops with short or strided pieces, zero fills, and whatever a bulk unit's
     //      addresses do not allow the TMA engine to take -------------------------------------------
-    const uint32_t w0 = warp - 1, nw = (blockDim.x >> 5) - 1;
-    for (uint64_t k = w0;; k += nw) {
-      const uint64_t w = blockIdx.x + k * (uint64_t)gridDim.x;
-      if (w >= simt_total) break;
-      uint64_t unit;
-      uint32_t layer;
-      split_unit(w, p.simt_units, &unit, &layer);
-      const Resolved r = resolve(p, simt_ops, p.n_simt_ops, unit, p.layer_begin + layer, lane == 0);
-      if (r.n != 0) warp_pieces(r, lane);
-    }
-    for (uint64_t k = w0;; k += nw) {
-      const uint64_t w = blockIdx.x + k * (uint64_t)gridDim.x;
-      if (w >= bulk_total) break;
-      uint64_t unit;
-      uint32_t layer;
-      split_unit(w, p.bulk_units, &unit, &layer);
-      const Resolved r = resolve(p, bulk_ops, p.n_bulk_ops, unit, p.layer_begin + layer, false);
-      if (r.n != 0 && !bulk_ok(r)) warp_pieces(r, lane);
-    }
+    simt_units(p, warp - 1, (blockDim.x >> 5) - 1, lane);
   }
 }
 
@@ -302,15 +348,15 @@ extern "C" int kvt_launch_walk(const KvtWalkLaunch* args, int grid_ctas, void* s
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 1;
-  // four CTAs per SM, each with two 8 KiB segments in flight through the TMA engine and seven SIMT warps.  Two
-  // stages, not four: 16 KiB of shared memory per CTA lets the CTAs of the next layer's launch start beside
-  // those of the running one (measured on the MLA step: 2495-2538 against 2225-2283 GB/s; three stages 2346,
-  // one 1905; the hybrid GDN step is the same within its run-to-run spread)
+  // Four CTAs per SM, each with three 8 KiB segments in the TMA engine and seven SIMT warps.  One launch of 61 MLA layers
+  // (10000 tokens, 961 MB read and written) takes 180 us with two stages, 168 with three, 167 with four; 12 hybrid GDN
+  // layers (1013 MB) 180 / 170 / 168; 5 requests of 600 MLA tokens 58.3 / 52.7 / 54.5.  More CTAs than are resident (1184
+  // to 4736) gain nothing there and cost 40 to 180 % on a launch of 63 MB.
   int grid = grid_ctas > 0 ? grid_ctas : 4 * sms;
   const uint64_t n_layers = a.layer_end - a.layer_begin;
   uint32_t threads = a.shape & 0xffffu, stages = a.shape >> 16;
   if (threads == 0) threads = 256;
-  if (stages == 0) stages = 2;
+  if (stages == 0) stages = 3;
   if (threads < 64 || threads > 256 || (threads & 31u) != 0 || stages > kMaxStagesW) return (int)cudaErrorInvalidValue;
   const uint64_t simt_warps = threads / 32 - 1;
   const uint64_t most = (a.bulk_units > a.simt_units / simt_warps ? a.bulk_units : (a.simt_units + simt_warps - 1) / simt_warps) * n_layers;
