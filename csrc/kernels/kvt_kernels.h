@@ -89,8 +89,9 @@ typedef struct KvtAttnLaunch {
   uint32_t* done_counter;      // device, zero before launch; may be NULL with flag == NULL
   uint64_t* flag;              // completion word (device / peer / host-mapped) or NULL
   uint64_t flag_value;         // value stored to *flag by the last CTA after a system fence
-  uint32_t simt_tile;          // SIMT path: 0 / 1 = a warp per tile (device destinations), 2 = a CTA per tile
-                               // (mapped host destinations: longer contiguous PCIe writes)
+  uint32_t simt_tile;          // who reads a tile where TMA does not copy it: 0 = the launcher's choice (fp8 -> bf16: the
+                               // bulk-fed expansion kernel, a local quantiser: four warps, else a warp), 1 = a warp, 4 =
+                               // four warps, 2 = a CTA (mapped host memory: longer contiguous PCIe writes)
   uint32_t dst_remote;         // 1: the destination is another GPU's memory.  The quantiser then stages its
                                // output in shared memory and sends it with bulk stores (256-byte NVLink
                                // packets); into local memory its own 16-byte stores are faster.

@@ -106,7 +106,7 @@ class AttnTransfer:
         self.src_kvt, self.dst_kvt = src_layout.to_kvt(), dst_layout.to_kvt()
         self.num_layers = len(src_ptrs)
         self.mode = mode
-        self.simt_tile = simt_tile      # 2: a CTA per tile (mapped host memory on the other side), else a warp per tile
+        self.simt_tile = simt_tile      # 2: a CTA per tile (mapped host memory on the other side), 0: the launcher's choice
         self.dst_remote = dst_remote    # the destination pointers are another GPU's memory (peer-mapped)
         self.head_map = head_map or HeadMap(0, 0, min(src_layout.num_heads, dst_layout.num_heads))
         import math

@@ -120,3 +120,45 @@ def test_tile_beyond_the_range_of_the_multiplied_division():
     pool, chunks = _chunks(random.Random(9), 256, [(0, 256), (2, 251)])
     a, b = (AttnLayout(s, pool, 256, 33, 128, 2) for s in (CacheShape.FLASH, CacheShape.FLASHINFER))
     _check(a, b, chunks, HeadMap(0, 0, 33), MODE_COPY, layers=1, use_tma=False)
+
+
+@pytest.mark.parametrize("mode", [MODE_BF16_TO_MXFP8, MODE_MXFP8_TO_BF16])
+@pytest.mark.parametrize("simt_tile", [0, 1, 2, 4])
+@pytest.mark.parametrize("heads, hm, tile_tokens, dst", [
+    (4, HeadMap(1, 2, 2), 16, CacheShape.FLASHINFER),     # a window of the heads: one run per head or token
+    (1, HeadMap(0, 0, 1), 1, CacheShape.FLASHINFER),      # single rows, scale runs of 4 bytes: read where they are
+    (3, HeadMap(0, 0, 3), 4, CacheShape.QWEN3_NEXT_FLASH),
+    (40, HeadMap(0, 0, 40), 16, CacheShape.FLASHINFER),   # tiles larger than a stage of the expansion kernel
+])
+def test_every_way_of_reading_a_tile_gives_the_same_bytes(heads, hm, tile_tokens, dst, simt_tile, mode):
+    pool, chunks = _chunks(random.Random(heads), 16, EDGES)
+    wide = AttnLayout(CacheShape.FLASH, pool, 16, heads, 128, 2)
+    mx = AttnLayout(dst, pool, 16, heads, 128, 1, mx_scaled=True)
+    a, b = (wide, mx) if mode == MODE_BF16_TO_MXFP8 else (mx, wide)
+
+    def prep(s):
+        s.bitwise_and_(0xF7)
+        mx.scale_view(s).copy_(torch.randint(100, 150, mx.scale_view(s).shape, dtype=torch.uint8, device=DEV))
+
+    _check(a, b, chunks, hm, mode, layers=1, prepare=prep if mode == MODE_MXFP8_TO_BF16 else None, tile_tokens=tile_tokens,
+           simt_tile=simt_tile)
+
+
+@pytest.mark.parametrize("mode", [MODE_COPY, MODE_MXFP8_TO_BF16])
+def test_more_tiles_than_the_grid_and_a_padded_tail(mode):
+    """A launch whose CTAs pass several tiles through their stages, with tail slots to zero behind a partly filled tile."""
+    pool, chunks = _chunks(random.Random(4), 16, [(5, 3000), (0, 4001), (16, 777)])
+    for c in chunks:
+        c.pad_tail = True
+    wide = AttnLayout(CacheShape.FLASH, pool, 16, 2, 128, 2)
+    mx = AttnLayout(CacheShape.FLASHINFER, pool, 16, 2, 128, 1, mx_scaled=True)
+    hnd = AttnLayout(CacheShape.FLASHINFER, pool, 16, 2, 128, 2)
+
+    def prep(s):
+        s.bitwise_and_(0xF7)
+        mx.scale_view(s).copy_(torch.randint(100, 150, mx.scale_view(s).shape, dtype=torch.uint8, device=DEV))
+
+    if mode == MODE_COPY:
+        _check(wide, hnd, chunks, HeadMap(0, 0, 2), mode, layers=3)
+    else:
+        _check(mx, wide, chunks, HeadMap(0, 0, 2), mode, layers=3, prepare=prep)
