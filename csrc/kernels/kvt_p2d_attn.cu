@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
       // from `flat` on.  A partly filled tile is LOADED whole: its other slots are cache memory of the same block, read
       // and dropped.
       struct Slot { const void* dmap; char* flat; int c1, c2, c3, c4; uint32_t lo, n; };
-      Slot slots[kMaxStages] = {};
+      Slot slots[kMaxStages];
       uint32_t issued = 0, stored = 0;
       bool failed = false;
       const bool token_inner = p.tile_order != 0u;
@@ -1248,16 +1248,19 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
   const uint32_t tile_bytes = tma ? a.src.head_bytes * a.n_heads * a.tile_tokens : 0u;
   int resident = grid;   // CTAs that are on the GPU together
   if (tma && grid_ctas <= 0 && a.dst_remote == 0 && tile_bytes != 0) {
-    // A long launch inside one GPU: CTAs of 128 KiB of tiles, handed to the SMs as they become free, six at a time on
-    // each.  With a fixed share for each of four CTAs per SM the slowest one ends the launch: 32 layers of 8192 tokens
-    // and 8 heads (1 GiB) took 361 us so and 341 with 3 to 4 tiles a CTA (343 with 7, 349 with 14); at 4 heads and
-    // 191 tiles a layer 77 us both ways, and 83 with one tile a CTA.  Over NVLink the link bounds either.
+    // Inside one GPU: as many CTAs per SM as have two tiles each in 200 KiB, 6 to 12.  One thread drives a CTA's tiles, so
+    // small ones want more CTAs: 500 tiles a layer of 4 KiB (1 head, 32 layers, 66 MB) 32.7 us with 4 or 6 a SM, 25 to 28 with
+    // 12 or 16; 80 layers 168 -> 142; 8 KiB tiles 189 -> 184; 32 KiB tiles (291 MB) 63.5 us with 4, 58.4 with 6.
+    const int per_sm = (int)std::min(12u, std::max(6u, kSmemBudget / 2u / tile_bytes));
+    grid = resident = per_sm * sms;
+    // A long launch: CTAs of 128 KiB of tiles, handed to the SMs as they become free.  With a fixed share for each the
+    // slowest one ends the launch: 32 layers of 8192 tokens and 8 heads (1 GiB) took 361 us so and 341 with 3 to 4 tiles a
+    // CTA (343 with 7, 349 with 14); at 4 heads and 191 tiles a layer 77 us both ways, and 83 with one tile a CTA.
+    // Over NVLink the link bounds either.
     const uint64_t tiles = tile_bytes < (128u << 10) ? (128u << 10) / tile_bytes : 1u;
     const uint64_t want = (total + tiles - 1) / tiles;
-    if (want > (uint64_t)grid) {
-      grid = (int)(want < (1u << 30) ? want : (1u << 30));
-      resident = grid < 6 * sms ? grid : 6 * sms;
-    }
+    if (want > (uint64_t)grid) grid = (int)(want < (1u << 30) ? want : (1u << 30));
+    if (threads <= 0) threads = 64;      // the second warp zeroes tails; 12 CTAs of 128 threads would not fit the registers
   }
   if ((uint64_t)grid > total) grid = (int)total;
   if (threads <= 0) threads = use_tma ? 128 : 512;
