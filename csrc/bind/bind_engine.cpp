@@ -190,7 +190,7 @@ KvTransferClient* need_client() {
 // One layer of the forward pass: its event on the engine's stream, and word of it to the open step.
 void record_layer(KvTransferClient* c, size_t stepid, uint64_t event, uint64_t stream) {
   cuda_check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "cudaEventRecord(layer)");
-  c->notify_event_record(stepid);
+  c->notify_event_record(stepid, stream);
 }
 
 std::optional<WorkerInfo> parse_py_worker_info(const py::handle& h) {

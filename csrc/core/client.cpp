@@ -304,9 +304,11 @@ size_t KvTransferClient::start_send(size_t stepid, size_t sched_tokens) {
   return stepid;
 }
 
-void KvTransferClient::notify_event_record(size_t step_id) {
+void KvTransferClient::notify_event_record(size_t step_id, std::optional<uint64_t> stream) {
   if (!last_step_guard_ || last_step_guard_->step_id() != step_id)
     throw KVTransferException(ErrorKind::INVALID_OPERATION, "event record before step start;");
+  if (stream.has_value()) last_step_guard_->step()->note_stream(*stream);
+  else last_step_guard_->step()->note_unknown_stream();
   last_step_guard_->after_record_one();
 }
 

@@ -57,7 +57,8 @@ class KvTransferClient {
   void submit_delta_send(const RequestId& reqid, uint32_t seen_tokens, uint32_t new_tokens, bool has_last_token,
                          size_t stepid, uint32_t substepid);
   size_t start_send(size_t stepid, size_t sched_tokens);
-  void notify_event_record(size_t step_id);
+  // `stream`: the raw handle the layer's event was recorded on; without it the layers count as recorded on several streams.
+  void notify_event_record(size_t step_id, std::optional<uint64_t> stream = std::nullopt);
   void flush_send(size_t step_id);
   void start_send_substep(size_t stepid, uint32_t substepid, std::vector<ReqMeta>& metas);  // thread safe
 

@@ -43,12 +43,22 @@ class Step {
   // wait-layers thread: true when all `layers` have been recorded before anybody wanted ready(i)
   bool all_recorded_unwanted(uint32_t layers) {
     return !ready_wanted_.load(std::memory_order_acquire) && record_signal_.wait_or(layers - 1, ready_wanted_) &&
-           !ready_wanted_.load(std::memory_order_acquire);
+           !ready_wanted_.load(std::memory_order_acquire) && one_stream();
   }
   uint32_t notify_layer_ready(uint32_t layers_done) { return data_signal_.release(layers_done); }
   void wait_layer_recorded(uint32_t layer) { record_signal_.wait(layer); }
   uint32_t notify_layer_recorded(uint32_t layers_recorded) { return record_signal_.release(layers_recorded); }
   void notify_one_recorded() { record_signal_.release(); }
+  // The raw handle of the stream that the next layer's event was recorded on, said before notify_one_recorded().  Only the
+  // engine thread calls it.
+  void note_stream(uint64_t stream) {
+    if (!stream_known_) stream_ = stream;
+    else if (stream != stream_) one_stream_.store(false, std::memory_order_release);
+    stream_known_ = true;
+  }
+  void note_unknown_stream() { one_stream_.store(false, std::memory_order_release); }
+  // True: the events of the layers recorded so far follow one another on one stream, so the last one implies the others.
+  bool one_stream() const { return one_stream_.load(std::memory_order_acquire); }
   uint32_t layers_recorded() { return record_signal_.value(); }
 
   Timepoint last_send_finish_ts() const noexcept { return Timepoint(SteadyClock::duration(last_send_finish_.load())); }
@@ -58,6 +68,9 @@ class Step {
   SyncSemaphore data_signal_;
   SyncSemaphore record_signal_;
   std::atomic<bool> ready_wanted_{false};
+  uint64_t stream_{0};
+  bool stream_known_{false};
+  std::atomic<bool> one_stream_{true};
   std::atomic<int64_t> last_send_finish_{0};
 };
 

@@ -106,3 +106,37 @@ def test_layers_recorded_on_the_current_stream_whichever_it_is():
         cli.drain()
         del cli
         srv.stop()
+
+
+@pytest.mark.parametrize("layers, tokens", [(6, 100), (9, 3001)])
+def test_layers_recorded_on_several_streams_of_one_step(layers, tokens):
+    """Even layers are produced late on one stream, odd ones at once on another: the event of the last layer of a launch says
+    nothing about the others."""
+    n = -(-tokens // BLOCK)
+    src, dst = _Cache(CacheShape.FLASH, layers, 2 * n + 2), _Cache(CacheShape.FLASH, layers, 2 * n + 2)
+    srv = KVTransferServer("D|0|1", 1, 0, 0, *dst.args, **dst.kw)
+    cli = KVTransferClient("P|0|1", 1, 0, 0, *src.args, **src.kw)
+    try:
+        slow, fast = torch.cuda.Stream(), torch.cuda.Stream()
+        big = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+        for step in (1, 2, 3):
+            cli.submit_req_send2("D|0|1", 0, "r%d" % step, 0, tokens, True, list(range(n)), list(range(n + 1, 2 * n + 1)),
+                                 srv.worker_info(), stepid=step)
+            cli.start_send_step(step, 1)
+            for layer in range(layers):
+                with torch.cuda.stream(fast if layer % 2 else slow):
+                    if layer % 2 == 0:
+                        for _ in range(4):
+                            big.fill_(layer)
+                    src.layers[layer][0].fill_(40 * step + layer)
+                    cli.record_event(layer)
+            cli.flush_send_step()
+            assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+            torch.cuda.synchronize()
+            for layer in range(layers):
+                got = dst.rows(layer, n + 1, n)[0][:tokens]
+                assert int(got.min()) == int(got.max()) == 40 * step + layer
+    finally:
+        cli.drain()
+        del cli
+        srv.stop()
