@@ -183,6 +183,17 @@ DeviceStage& BatchEngine::stage(size_t i) {
   return *stages_[i];
 }
 
+void* BatchEngine::launch_stream(size_t stage_idx, void* wait_event) {
+  if (stage_idx == kSlotStream) {
+    cudaStream_t s = cur().stream;
+    if (wait_event != nullptr) cuda_check(cudaStreamWaitEvent(s, static_cast<cudaEvent_t>(wait_event), 0), "cudaStreamWaitEvent");
+    return s;
+  }
+  DeviceStage& st = stage(stage_idx);
+  st.wait_event(wait_event);
+  return st.stream();
+}
+
 int BatchEngine::grid() const {
   if (cfg_.grid_ctas > 0) return cfg_.grid_ctas;
   return std::max(1, static_cast<int>(4 * kvt_sm_count(cfg_.device) * env_kernel_copy_sm_usage()));
@@ -238,8 +249,7 @@ void BatchEngine::launch_attn(const DeviceAttnParams& params, const PackedPlan& 
   if (plan.n_reqs == 0 || hi <= lo) return;
   cuda_check(cudaSetDevice(cfg_.device), "cudaSetDevice");
   ensure_attn_arrays(params);
-  DeviceStage& st = stage(stage_idx);
-  if (wait_event != nullptr) st.wait_event(wait_event);
+  void* stream = launch_stream(stage_idx, wait_event);
   Slot& sl = cur();
   KvtAttnLaunch a{};
   a.src_layers = d_src_layers_.p;
@@ -263,7 +273,7 @@ void BatchEngine::launch_attn(const DeviceAttnParams& params, const PackedPlan& 
   a.dst_remote = cfg_.dst_remote ? 1u : 0u;
   a.tile_order = tile_order_;
   a.store_form = store_form_;
-  cuda_check(kvt_launch_p2d_attn(&a, cfg_.one_gpu && cfg_.grid_ctas <= 0 && env_kernel_copy_sm_usage() >= 1.0 ? 0 : grid(), 0, use_tma_ ? 1 : 0, st.stream()), "kvt_launch_p2d_attn");
+  cuda_check(kvt_launch_p2d_attn(&a, cfg_.one_gpu && cfg_.grid_ctas <= 0 && env_kernel_copy_sm_usage() >= 1.0 ? 0 : grid(), 0, use_tma_ ? 1 : 0, stream), "kvt_launch_p2d_attn");
 }
 
 void BatchEngine::ensure_walk_arrays() {
@@ -281,8 +291,7 @@ void BatchEngine::launch_walk(const KvtWalkCounts& c, size_t n_ops, size_t pool_
   if (n_ops == 0 || hi <= lo) return;
   cuda_check(cudaSetDevice(cfg_.device), "cudaSetDevice");
   ensure_walk_arrays();
-  DeviceStage& st = stage(stage_idx);
-  if (wait_event != nullptr) st.wait_event(wait_event);
+  void* stream = launch_stream(stage_idx, wait_event);
   Slot& sl = cur();
   KvtWalkLaunch a{};
   a.src_ptrs = d_walk_src_.p;
@@ -304,7 +313,7 @@ void BatchEngine::launch_walk(const KvtWalkCounts& c, size_t n_ops, size_t pool_
   a.pool = reinterpret_cast<const uint32_t*>(sl.d_plan + n_ops * sizeof(KvtWalkOp));
   a.pool_len = static_cast<uint32_t>(pool_len);
   a.status = sl.d_status;
-  if (a.n_bulk_ops + a.n_simt_ops != 0) cuda_check(kvt_launch_walk(&a, grid(), st.stream()), "kvt_launch_walk");
+  if (a.n_bulk_ops + a.n_simt_ops != 0) cuda_check(kvt_launch_walk(&a, grid(), stream), "kvt_launch_walk");
   if (c.n_zero != 0) {
     // tail padding lands after the copies (same stream): where both touch a byte, the zero wins, as it does
     // when the byte ranges are applied in the planner's order
@@ -313,7 +322,7 @@ void BatchEngine::launch_walk(const KvtWalkCounts& c, size_t n_ops, size_t pool_
     a.bulk_units = 0;
     a.n_simt_ops = c.n_zero;
     a.simt_units = c.zero_units;
-    cuda_check(kvt_launch_walk(&a, grid(), st.stream()), "kvt_launch_walk(zero fill)");
+    cuda_check(kvt_launch_walk(&a, grid(), stream), "kvt_launch_walk(zero fill)");
   }
 }
 

@@ -67,6 +67,11 @@ class BatchEngine {
   bool in_batch() const { return batch_slot_ >= 0; }
   // Transfer stream `i` of the current batch (joined to the plan upload at first use).
   DeviceStage& stage(size_t i);
+  // As a stage index: the slot's own stream.  Its launches need no event behind the upload and none in front of the
+  // completion record, and run one after the other.
+  static constexpr size_t kSlotStream = SIZE_MAX;
+  // The stream that stage's next launch goes to, made to wait for the plan's upload and for `wait_event` (nullptr: none).
+  void* launch_stream(size_t stage_idx, void* wait_event);
   size_t n_stages() const { return stages_.size(); }
   size_t next_stage() { return range_rr_++ % stages_.size(); }
 
