@@ -90,7 +90,7 @@ typedef struct KvtAttnLaunch {
   uint64_t* flag;              // completion word (device / peer / host-mapped) or NULL
   uint64_t flag_value;         // value stored to *flag by the last CTA after a system fence
   uint32_t simt_tile;          // who reads a tile where TMA does not copy it: 0 = the launcher's choice (fp8 -> bf16: the
-                               // bulk-fed expansion kernel, a local quantiser: four warps, else a warp), 1 = a warp, 4 =
+                               // bulk-fed expansion kernel, a local quantiser: four warps, small tiles: a warp), 1 = a warp, 4 =
                                // four warps, 2 = a CTA (mapped host memory: longer contiguous PCIe writes)
   uint32_t dst_remote;         // 1: the destination is another GPU's memory.  The quantiser then stages its
                                // output in shared memory and sends it with bulk stores (256-byte NVLink

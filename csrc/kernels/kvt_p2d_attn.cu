@@ -1088,14 +1088,15 @@ bool quant_staged(const KvtAttnLaunch& a) {
   return stage_env > 0 || (stage_env < 0 && a.dst_remote != 0);
 }
 
-// The expansion kernel serves what leaves the way of reading open (simt_tile 0), in tiles of which kConvCtas fit an SM; for
-// the rest it says cudaErrorNotSupported and the SIMT kernel serves it.
+// The expansion kernel serves what leaves the way of reading open (simt_tile 0), in tiles of at least 4 KiB of codes (with
+// 2 KiB, one head, the hand-over of a tile costs more than its reading: 32 layers of 6000 tokens 51 us against 43) of which
+// kConvCtas fit an SM; for the rest it says cudaErrorNotSupported and the SIMT kernel serves it.
 cudaError_t launch_expand(const KvtAttnLaunch& a, int grid_ctas, int sms, uint64_t total, cudaStream_t stream) {
   const uint64_t rows = (uint64_t)a.n_heads * a.tile_tokens;
   const uint64_t tile_bytes = (rows * a.src.head_bytes + 127u) & ~127ull;
   const uint64_t stage_bytes = tile_bytes + ((rows * (a.src.head_bytes >> 5) + 127u) & ~127ull);
   const uint64_t budget = kSmemBudget / kConvCtas;
-  if (simt_choice(a) != 0 || a.dst_remote != 0 || stage_bytes > budget) return cudaErrorNotSupported;
+  if (simt_choice(a) != 0 || a.dst_remote != 0 || tile_bytes < 4096u || stage_bytes > budget) return cudaErrorNotSupported;
   uint64_t stages = budget / stage_bytes;
   if (stages > (uint64_t)kConvStages) stages = kConvStages;
   uint64_t grid = (uint64_t)grid_ctas;
@@ -1121,10 +1122,11 @@ cudaError_t launch_impl(const KvtAttnLaunch& a, int grid, int threads, uint32_t 
   } else if (choice == 1 || (choice == 4 && threads % 128 == 0)) {
     warp_tiles = (uint32_t)choice;
   } else {
-    // Four warps share a tile of the local quantiser, so that more of it is in flight at once: 80 layers of 376 tiles of
-    // 2 heads 158 us against 159 with a warp per tile, 32 layers of 500 tiles of 8 heads 283 against 307 (5.6 TB/s).  The
-    // staged form (remote destinations) and the host-side copies keep a tile with one warp.
-    warp_tiles = MODE == KVT_MODE_BF16_TO_MXFP8 && threads % 128 == 0 && !quant_staged(a) ? 4u : 1u;
+    // Four warps share a tile of 16 KiB or more of the local quantiser, so that more of it is in flight at once: 32 layers
+    // of 500 tiles of 8 heads 283 us against 307 with a warp per tile (5.6 TB/s), 2 heads (8 KiB) 158 against 159, one head
+    // 57 against 45.  The staged form (remote destinations) and the host-side copies keep a tile with one warp.
+    const uint64_t tile = (uint64_t)a.n_heads * a.tile_tokens * a.src.head_bytes;
+    warp_tiles = MODE == KVT_MODE_BF16_TO_MXFP8 && threads % 128 == 0 && tile >= 16384u && !quant_staged(a) ? 4u : 1u;
   }
   if (!USE_TMA && warp_tiles != 0u) {
     const uint64_t owners = warps / warp_tiles;

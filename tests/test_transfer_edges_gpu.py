@@ -128,6 +128,8 @@ def test_tile_beyond_the_range_of_the_multiplied_division():
     (4, HeadMap(1, 2, 2), 16, CacheShape.FLASHINFER),     # a window of the heads: one run per head or token
     (1, HeadMap(0, 0, 1), 1, CacheShape.FLASHINFER),      # single rows, scale runs of 4 bytes: read where they are
     (3, HeadMap(0, 0, 3), 4, CacheShape.QWEN3_NEXT_FLASH),
+    (4, HeadMap(0, 0, 4), 16, CacheShape.QWEN3_NEXT_FLASH),   # scale bytes of a head apart: read where they are
+    (16, HeadMap(0, 0, 16), 4, CacheShape.FLASHINFER),    # a run of four rows and one of 16 scale bytes per head
     (40, HeadMap(0, 0, 40), 16, CacheShape.FLASHINFER),   # tiles larger than a stage of the expansion kernel
 ])
 def test_every_way_of_reading_a_tile_gives_the_same_bytes(heads, hm, tile_tokens, dst, simt_tile, mode):
