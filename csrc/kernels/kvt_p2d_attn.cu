@@ -1250,10 +1250,11 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
   const uint32_t tile_bytes = tma ? a.src.head_bytes * a.n_heads * a.tile_tokens : 0u;
   int resident = grid;   // CTAs that are on the GPU together
   if (tma && grid_ctas <= 0 && a.dst_remote == 0 && tile_bytes != 0) {
-    // Inside one GPU: as many CTAs per SM as have two tiles each in 200 KiB, 6 to 12.  One thread drives a CTA's tiles, so
+    // Inside one GPU: as many CTAs per SM as have two tiles each in 200 KiB, 4 to 12.  One thread drives a CTA's tiles, so
     // small ones want more CTAs: 500 tiles a layer of 4 KiB (1 head, 32 layers, 66 MB) 32.7 us with 4 or 6 a SM, 25 to 28 with
-    // 12 or 16; 80 layers 168 -> 142; 8 KiB tiles 189 -> 184; 32 KiB tiles (291 MB) 63.5 us with 4, 58.4 with 6.
-    const int per_sm = (int)std::min(12u, std::max(6u, kSmemBudget / 2u / tile_bytes));
+    // 12 or 16; 80 layers 168 -> 142; 8 KiB tiles 189 -> 184.  32 KiB tiles keep 4: a lone launch of 291 MB takes
+    // 63.5 us so and 58.4 with 6, but one-layer launches of 1024 tiles overlapping on 8 streams 3172 and 2966 GB/s.
+    const int per_sm = (int)std::min(12u, std::max(4u, kSmemBudget / 2u / tile_bytes));
     grid = resident = per_sm * sms;
     // A long launch: CTAs of 128 KiB of tiles, handed to the SMs as they become free.  With a fixed share for each the
     // slowest one ends the launch: 32 layers of 8192 tokens and 8 heads (1 GiB) took 361 us so and 341 with 3 to 4 tiles a
@@ -1261,7 +1262,10 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
     // Over NVLink the link bounds either.
     const uint64_t tiles = tile_bytes < (128u << 10) ? (128u << 10) / tile_bytes : 1u;
     const uint64_t want = (total + tiles - 1) / tiles;
-    if (want > (uint64_t)grid) grid = (int)(want < (1u << 30) ? want : (1u << 30));
+    if (want > (uint64_t)grid) {
+      grid = (int)(want < (1u << 30) ? want : (1u << 30));
+      resident = std::max(resident, std::min(grid, 6 * sms));
+    }
     if (threads <= 0) threads = 64;      // the second warp zeroes tails; 12 CTAs of 128 threads would not fit the registers
   }
   if ((uint64_t)grid > total) grid = (int)total;
