@@ -865,11 +865,16 @@ struct ConvSlot {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// The calling lane's wait.  Lanes read their own clocks, so at the limit some may give up where others were served.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity))
     if (clock64() - t0 > kWaitCycles) return false;
   return true;
+}
+// The wait of a whole warp, with one outcome for all of its lanes: they go on, or leave, together.
+__device__ __forceinline__ bool warp_wait_bounded(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity)) != 0;
 }
 __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
@@ -918,8 +923,8 @@ __global__ void __launch_bounds__(kConvThreads, kConvCtas) kvt_p2d_expand_kernel
     // the next stage, free again (its converting warps are bounded in their own waits)
     auto acquire = [&]() {
       const uint32_t s = issued % n_stages;
-      if (issued >= n_stages && !mbar_wait_bounded(smem_u32(&empty[s]), (issued / n_stages - 1u) & 1u)) {
-        set_status(p.status, KVT_ERR_TMA_TIMEOUT, issued);
+      if (issued >= n_stages && !warp_wait_bounded(smem_u32(&empty[s]), (issued / n_stages - 1u) & 1u)) {
+        if (lane == 0) set_status(p.status, KVT_ERR_TMA_TIMEOUT, issued);
         failed = true;
       }
       ++issued;
@@ -1005,9 +1010,9 @@ __global__ void __launch_bounds__(kConvThreads, kConvCtas) kvt_p2d_expand_kernel
     for (uint32_t k = 0;; ++k) {
       const uint32_t s = k % n_stages;
       const uint32_t bar = smem_u32(&full[s]), parity = (k / n_stages) & 1u;
-      if (!mbar_wait_bounded(bar, parity)) {
-        set_status(p.status, KVT_ERR_TMA_TIMEOUT, k);
-        mbar_wait_bounded(bar, parity);      // copies may still be on their way into this CTA's shared memory
+      if (!warp_wait_bounded(bar, parity)) {
+        if (lane == 0) set_status(p.status, KVT_ERR_TMA_TIMEOUT, k);
+        warp_wait_bounded(bar, parity);      // copies may still be on their way into this CTA's shared memory
         break;
       }
       const TileMove m = slots[s].move;

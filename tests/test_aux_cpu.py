@@ -1,8 +1,10 @@
 """Auxiliary subsystems on CPU: process monitor line protocol, gdrcopy shim, CRC, NVLink affinity
 table helpers, KV specs of the model families."""
 import os
+import re
 import socket
 import zlib
+from pathlib import Path
 
 from llumnix_kv_b200 import load_ops, nvlink_affinity
 from llumnix_kv_b200.models.kv_spec import DEEPSEEK_V32, LLAMA3_8B, LLAMA3_70B, QWEN3_NEXT_80B, SPECS
@@ -209,3 +211,19 @@ def test_crash_trace_prints_native_frames_then_chains(ops):
     assert r.returncode == -11, (r.returncode, r.stderr[-500:])
     assert "kvtransfer crash trace: signal 11" in r.stderr and "end of trace" in r.stderr
     assert "(+0x" in r.stderr or "[0x" in r.stderr
+
+
+def test_a_bounded_wait_of_a_warp_has_one_outcome_for_its_lanes():
+    """Lanes that read their own clocks may disagree at the limit; where some left a loop that the others' shuffles and warp
+    barriers go on in, the warp would wait for lanes that have gone.  So every wait in the kernels is either lane 0's alone or
+    goes through a vote."""
+    text = (Path(__file__).parent.parent / "csrc" / "kernels" / "kvt_p2d_attn.cu").read_text()
+    vote = re.search(r"bool warp_wait_bounded\(.*?\n}\n", text, re.S)
+    assert vote is not None and "__all_sync(0xffffffffu, mbar_wait_bounded(" in vote.group(0)
+    definition = re.search(r"bool mbar_wait_bounded\(.*?\n}\n", text, re.S).group(0)
+    rest = text.replace(vote.group(0), "").replace(definition, "")
+    assert "mbar_wait_bounded(" not in rest.replace("warp_wait_bounded(", "")
+    for use in re.finditer(r"(?<![a-z_])mbar_try_wait\(bar, parity\)", rest):
+        # what is left: the copy kernel's pipeline, which one lane drives
+        assert rest.rindex("auto consume_one = [&]", 0, use.start()) > rest.rindex("__global__", 0, use.start())
+    assert "if (lane == 0 && !failed) {" in rest and "while (!failed && stored < issued) consume_one();" in rest
