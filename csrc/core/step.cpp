@@ -44,7 +44,7 @@ void StepGuard::wait_layers() {
   uint32_t val = step_->notify_layer_ready(0);
   if (val > 0) return;  // a frozen step: born with every layer ready
   for (uint32_t layer = 0; layer < num_layers; ++layer) {
-    if (step_->all_recorded_unwanted(num_layers)) layer = num_layers - 1;   // one stream: the last event implies all
+    if (step_->all_recorded_unwanted(num_layers)) layer = num_layers - 1;
     step_->wait_layer_recorded(layer);
     barrier_->wait(layer);
     val = step_->notify_layer_ready(layer + 1);

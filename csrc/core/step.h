@@ -40,10 +40,11 @@ class Step {
   void want_ready() {
     if (!ready_wanted_.exchange(true, std::memory_order_acq_rel)) record_signal_.kick();
   }
-  // wait-layers thread: true when all `layers` have been recorded before anybody wanted ready(i)
+  // wait-layers thread: true when all `layers` have been recorded before anybody wanted ready(i), and the last of their
+  // events implies the others
   bool all_recorded_unwanted(uint32_t layers) {
     return !ready_wanted_.load(std::memory_order_acquire) && record_signal_.wait_or(layers - 1, ready_wanted_) &&
-           !ready_wanted_.load(std::memory_order_acquire) && one_stream();
+           !ready_wanted_.load(std::memory_order_acquire) && last_event_implies(layers);
   }
   uint32_t notify_layer_ready(uint32_t layers_done) { return data_signal_.release(layers_done); }
   void wait_layer_recorded(uint32_t layer) { record_signal_.wait(layer); }
@@ -52,13 +53,16 @@ class Step {
   // The raw handle of the stream that the next layer's event was recorded on, said before notify_one_recorded().  Only the
   // engine thread calls it.
   void note_stream(uint64_t stream) {
-    if (!stream_known_) stream_ = stream;
-    else if (stream != stream_) one_stream_.store(false, std::memory_order_release);
-    stream_known_ = true;
+    const uint32_t n = in_line_.load(std::memory_order_relaxed);
+    if (n == 0) stream_ = stream;
+    if (stream != stream_) out_of_line_ = true;
+    if (!out_of_line_) in_line_.store(n + 1, std::memory_order_release);
   }
-  void note_unknown_stream() { one_stream_.store(false, std::memory_order_release); }
-  // True: the events of the layers recorded so far follow one another on one stream, so the last one implies the others.
-  bool one_stream() const { return one_stream_.load(std::memory_order_acquire); }
+  void note_unknown_stream() { out_of_line_ = true; }
+  // True: the events of layers [0, layers) were all recorded in this step and follow one another on one stream, so that the
+  // last one implies the others.  False where that is not known: after a flush that came before the last layer's record, the
+  // event of a layer that was not recorded is one of an earlier step and says nothing about this one.
+  bool last_event_implies(size_t layers) const { return in_line_.load(std::memory_order_acquire) >= layers; }
   uint32_t layers_recorded() { return record_signal_.value(); }
 
   Timepoint last_send_finish_ts() const noexcept { return Timepoint(SteadyClock::duration(last_send_finish_.load())); }
@@ -69,8 +73,8 @@ class Step {
   SyncSemaphore record_signal_;
   std::atomic<bool> ready_wanted_{false};
   uint64_t stream_{0};
-  bool stream_known_{false};
-  std::atomic<bool> one_stream_{true};
+  bool out_of_line_{false};             // engine thread: a layer came on another stream, or on one that was not named
+  std::atomic<uint32_t> in_line_{0};    // leading layers noted on one stream
   std::atomic<int64_t> last_send_finish_{0};
 };
 

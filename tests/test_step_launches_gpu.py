@@ -140,3 +140,42 @@ def test_layers_recorded_on_several_streams_of_one_step(layers, tokens):
         cli.drain()
         del cli
         srv.stop()
+
+
+@pytest.mark.parametrize("proto", [PT.NVLINK, PT.SHM])
+@pytest.mark.parametrize("shape", [CacheShape.FLASH, CacheShape.DPSK_V32_SPARSE_MLA])
+@pytest.mark.parametrize("recorded", [1, 5])
+def test_a_step_flushed_before_its_last_layers_still_waits_for_those_recorded(recorded, shape, proto):
+    """The layers behind the last one recorded keep the events (and the bytes) of the step before: those events are long
+    complete and say nothing about the layers that this step recorded."""
+    layers, n = 9, 3
+    src, dst = _Cache(shape, layers, 2 * n + 2), _Cache(shape, layers, 2 * n + 2)
+    args = lambda c: c.args[:4] + ([proto],)  # noqa: E731
+    srv = KVTransferServer("D|0|1", 1, 0, 0, *args(dst), **dst.kw)
+    cli = KVTransferClient("P|0|1", 1, 0, 0, *args(src), **src.kw)
+    try:
+        fwd = torch.cuda.Stream()
+        big = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+        value = [0] * layers
+        for step, upto in ((1, layers), (2, recorded), (3, recorded), (4, layers), (5, recorded)):
+            cli.submit_req_send2("D|0|1", 0, "r%d" % step, 0, n * BLOCK, True, list(range(n)), list(range(n + 1, 2 * n + 1)),
+                                 srv.worker_info(), stepid=step)
+            cli.start_send_step(step, 1)
+            with torch.cuda.stream(fwd):
+                for layer in range(upto):
+                    for _ in range(4):
+                        big.fill_(layer)
+                    value[layer] = 20 * step + layer
+                    for t in src.layers[layer]:
+                        t.fill_(value[layer])
+                    cli.record_event(layer)
+            cli.flush_send_step()
+            assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+            torch.cuda.synchronize()
+            for layer in range(layers):
+                for got in dst.rows(layer, n + 1, n):
+                    assert int(got.min()) == int(got.max()) == value[layer], (step, layer)
+    finally:
+        cli.drain()
+        del cli
+        srv.stop()
