@@ -177,6 +177,7 @@ void KvTransferClient::start_req_send(std::vector<ReqMeta>& metas, size_t stepid
   auto step = std::make_shared<Step>(stepid);
   // the data is complete: the step is born with every layer recorded and ready
   step->frozen = true;
+  if (events_in_line_.load(std::memory_order_acquire)) step->take_in_line(static_cast<uint32_t>(ctx_->num_layers()));
   step->notify_layer_recorded(ctx_->num_layers());
   step->notify_layer_ready(ctx_->num_layers());
   step->flush_send_ts = step->wait_layers_start_ts = step->wait_layers_end_ts = step->start_send_ts;
@@ -269,6 +270,7 @@ void KvTransferClient::start_send_substep(size_t stepid, uint32_t substepid, std
 size_t KvTransferClient::start_send(size_t stepid, size_t sched_tokens) {
   if (sched_tokens == 0 && pending_buf_.empty()) return EMPTY_STEP_ID;
   fault_inject_sleep(777 * 1000);
+  if (last_step_guard_) settle_events(*last_step_guard_->step());   // replaced without a flush
   auto step = std::make_shared<Step>(stepid);
   auto guard = std::make_shared<StepGuard>(ctx_.get(), step);
   wait_pool_->spawn([guard] {
@@ -312,9 +314,17 @@ void KvTransferClient::notify_event_record(size_t step_id, std::optional<uint64_
   last_step_guard_->after_record_one();
 }
 
+// A step closes: whether the last layer's event still implies those of all layers for who comes later.  A step that recorded
+// nothing leaves the events, and so the answer, as they were.
+void KvTransferClient::settle_events(Step& step) {
+  if (step.layers_recorded() != 0)
+    events_in_line_.store(step.last_event_implies(ctx_->num_layers()), std::memory_order_release);
+}
+
 void KvTransferClient::flush_send(size_t step_id) {
   if (!last_step_guard_ || last_step_guard_->step_id() != step_id)
     throw KVTransferException(ErrorKind::INVALID_OPERATION, "event record before step start;");
+  settle_events(*last_step_guard_->step());
   last_step_guard_->layer_ready_all();
   last_step_guard_->step()->flush_send_ts = SteadyClock::now();
   std::lock_guard<std::mutex> g(coord_lock_);

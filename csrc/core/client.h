@@ -105,6 +105,9 @@ class KvTransferClient {
   std::unordered_map<RequestId, std::vector<std::shared_ptr<RequestInfo>>> reqs_;
   StepTasks pending_buf_;  // chunks submitted for the next start_send (substep 0)
   TargetMgr mgr_;
+  // What the steps closed so far say about the events that a frozen step is ordered behind (engine thread writes).
+  std::atomic<bool> events_in_line_{true};
+  void settle_events(Step& step);
   std::mutex coord_lock_;
   size_t coord_step_id_{0};
   std::shared_ptr<StepGuard> last_step_guard_;

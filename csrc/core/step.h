@@ -59,8 +59,10 @@ class Step {
     if (!out_of_line_) in_line_.store(n + 1, std::memory_order_release);
   }
   void note_unknown_stream() { out_of_line_ = true; }
-  // True: the events of layers [0, layers) were all recorded in this step and follow one another on one stream, so that the
-  // last one implies the others.  False where that is not known: after a flush that came before the last layer's record, the
+  // A frozen step records nothing itself: the events it is ordered behind are those of the steps before it.
+  void take_in_line(uint32_t layers) { in_line_.store(layers, std::memory_order_release); }
+  // True: the events of layers [0, layers) were all recorded in this step (for a frozen step: in the last one that recorded
+  // any) and follow one another on one stream, so that the last one implies the others.  False where that is not known: after a flush that came before the last layer's record, the
   // event of a layer that was not recorded is one of an earlier step and says nothing about this one.
   bool last_event_implies(size_t layers) const { return in_line_.load(std::memory_order_acquire) >= layers; }
   uint32_t layers_recorded() { return record_signal_.value(); }

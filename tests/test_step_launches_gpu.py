@@ -8,7 +8,7 @@ import torch
 
 os.environ.setdefault("BLLM_KVTRANS_QUIET_ENV", "1")
 
-from llumnix_kv_b200.kv_transfer_impl import KVTransferClient, KVTransferProtocolType as PT, KVTransferServer
+from llumnix_kv_b200.kv_transfer_impl import KVTransferClient, KVTransferProtocolType as PT, KVTransferServer, ReqMeta
 from llumnix_kv_b200.ops.layouts import AttnLayout, CacheShape
 
 pytestmark = pytest.mark.gpu
@@ -174,6 +174,47 @@ def test_a_step_flushed_before_its_last_layers_still_waits_for_those_recorded(re
             torch.cuda.synchronize()
             for layer in range(layers):
                 for got in dst.rows(layer, n + 1, n):
+                    assert int(got.min()) == int(got.max()) == value[layer], (step, layer)
+    finally:
+        cli.drain()
+        del cli
+        srv.stop()
+
+
+@pytest.mark.parametrize("shape", [CacheShape.FLASH, CacheShape.DPSK_V32_SPARSE_MLA])
+@pytest.mark.parametrize("layers, blocks", [(9, 30), (34, 70)])
+def test_a_frozen_send_waits_for_the_layers_of_the_step_before_it(layers, blocks, shape):
+    """The step that produced the data used two streams, or recorded some of the layers only.  (34, 70) is 595 MiB of
+    the attention cache and goes out in several launches, the others in one."""
+    src, dst = _Cache(shape, layers, blocks + 1), _Cache(shape, layers, blocks + 1)
+    srv = KVTransferServer("D|0|1", 1, 0, 0, *dst.args, **dst.kw)
+    cli = KVTransferClient("P|0|1", 1, 0, 0, *src.args, **src.kw)
+    try:
+        slow, fast = torch.cuda.Stream(), torch.cuda.Stream()
+        big = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+        value = [0] * layers
+        # (streams of even and odd layers, layers recorded)
+        for step, (even, upto) in enumerate([(slow, layers), (fast, layers), (slow, layers), (fast, layers - 2), (slow, layers)], 1):
+            cli.start_send_step(step, 1)
+            for layer in range(upto):
+                with torch.cuda.stream(fast if layer % 2 else even):
+                    if layer % 2 == 0:
+                        for _ in range(4):
+                            big.fill_(layer)
+                    value[layer] = 40 * step + layer
+                    for t in src.layers[layer]:
+                        t.fill_(value[layer])
+                    cli.record_event(layer)
+            cli.flush_send_step()
+            m = ReqMeta()
+            m.dst_inst, m.dst_worker, m.reqid, m.dst_worker_info = "D|0|1", 0, "m%d" % step, srv.worker_info()
+            m.seen_tokens, m.new_tokens = 0, blocks * BLOCK
+            m.src_block_ids, m.dst_block_ids = [list(range(blocks))], [list(range(1, blocks + 1))]
+            cli.start_req_send([m], step)
+            assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+            torch.cuda.synchronize()
+            for layer in range(layers):
+                for got in dst.rows(layer, 1, blocks):
                     assert int(got.min()) == int(got.max()) == value[layer], (step, layer)
     finally:
         cli.drain()
