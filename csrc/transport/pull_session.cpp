@@ -100,21 +100,28 @@ void PullSession::on_plan(uint64_t seq, const char* body, size_t len) {
 void PullSession::on_layers(uint64_t seq, const char* body, size_t len) {
   if (seq != cur_seq_ || !have_batch_ || !error_.empty()) return;
   uint32_t lo = 0, hi = 0;
-  uint8_t one_launch = 0;
+  uint8_t flags = 0;
   const char* p = body;
   const char* end = body + len;
-  if (!take(p, end, &lo) || !take(p, end, &hi) || !take(p, end, &one_launch) || hi > events_.size() || lo >= hi) {
+  if (!take(p, end, &lo) || !take(p, end, &hi) || !take(p, end, &flags) || hi > events_.size() || lo >= hi) {
     error_ = "bad layers message";
     return;
   }
+  // a launch of several layers waits for the last of their events, and for the others where that does not imply them
+  auto order_behind = [&](size_t stage) {
+    if ((flags & PULL_LAYERS_EACH_EVENT) != 0)
+      for (uint32_t l = lo; l + 1 < hi; ++l) eng_->launch_stream(stage, events_[l]);
+  };
   try {
     if (head_.kind == PULL_KIND_WALK) {
-      // one launch for the range, behind the last of its layer events (recorded in order on one stream)
+      // one launch for the range
       const size_t stage = eng_->next_stage();
+      order_behind(stage);
       eng_->launch_walk(head_.walk, head_.n_ops, head_.pool_len, lo, hi, stage, events_[hi - 1]);
       // the bytes are here: the switch delivers them to the other members of the group from this GPU
       if (head_.fanout != 0) eng_->launch_walk_fanout(head_.walk, head_.n_ops, head_.pool_len, lo, hi, stage);
-    } else if (one_launch) {
+    } else if ((flags & PULL_LAYERS_ONE_LAUNCH) != 0) {
+      order_behind(0);
       eng_->launch_attn(head_.attn, attn_plan_, lo, hi, 0, events_[hi - 1]);
     } else {
       for (uint32_t l = lo; l < hi; ++l) eng_->launch_attn(head_.attn, attn_plan_, l, l + 1, l % eng_->n_stages(), events_[l]);

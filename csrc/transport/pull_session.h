@@ -36,8 +36,11 @@ struct PullPlanHead {
   DeviceAttnParams attn;
 };
 
+// Flags of a layers message: all of its layers in one launch; the last layer's event does not imply the others'.
+constexpr uint8_t PULL_LAYERS_ONE_LAUNCH = 1, PULL_LAYERS_EACH_EVENT = 2;
+
 inline uint32_t pull_protocol_version() {
-  return static_cast<uint32_t>(sizeof(PullPlanHead) ^ (sizeof(KvtWalkOp) << 12) ^ (sizeof(KvtReqDesc) << 24)) ^ 0x20250001u;
+  return static_cast<uint32_t>(sizeof(PullPlanHead) ^ (sizeof(KvtWalkOp) << 12) ^ (sizeof(KvtReqDesc) << 24)) ^ 0x20250002u;
 }
 
 class PullSession : public std::enable_shared_from_this<PullSession> {

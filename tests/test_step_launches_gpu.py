@@ -1,6 +1,8 @@
 """Several layers of a step in one launch: whatever the launches hold, every layer's bytes are those that the forward stream wrote
 before it recorded the layer's event, and nothing outside the request's slots is written."""
 import os
+import subprocess
+import sys
 import time
 
 import pytest
@@ -216,6 +218,58 @@ def test_a_frozen_send_waits_for_the_layers_of_the_step_before_it(layers, blocks
             for layer in range(layers):
                 for got in dst.rows(layer, 1, blocks):
                     assert int(got.min()) == int(got.max()) == value[layer], (step, layer)
+    finally:
+        cli.drain()
+        del cli
+        srv.stop()
+
+
+@pytest.mark.parametrize("walk", [1, 0])
+def test_walk_and_descriptor_launches_of_layers_recorded_on_several_streams(walk):
+    """The two ways of moving a cache of several tensors a layer; the switch between them is read once in a process."""
+    script = """
+import torch
+import test_step_launches_gpu as t
+t.several_streams(t.CacheShape.DPSK_V32_SPARSE_MLA, 9, 3001)
+print("ok")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, BLLM_KVTRANS_NVLINK_WALK=str(walk), PYTHONPATH=os.pathsep.join([root, os.path.join(root, "tests")]))
+    r = subprocess.run([sys.executable, "-c", script], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.endswith("ok\n"), r.stderr[-3000:]
+
+
+def several_streams(shape, layers, tokens):
+    """Even layers late on one stream, odd ones at once on another.  The request joins the step when all of them have been
+    recorded, so that every launch takes as many as it can."""
+    n = -(-tokens // BLOCK)
+    src, dst = _Cache(shape, layers, n + 1), _Cache(shape, layers, n + 1)
+    srv = KVTransferServer("D|0|1", 1, 0, 0, *dst.args, **dst.kw)
+    cli = KVTransferClient("P|0|1", 1, 0, 0, *src.args, **src.kw)
+    try:
+        slow, fast = torch.cuda.Stream(), torch.cuda.Stream()
+        big = torch.empty(1 << 30, dtype=torch.uint8, device=DEV)
+        for step in (1, 2, 3):
+            cli.start_send_step(step, 1)
+            for layer in range(layers):
+                with torch.cuda.stream(fast if layer % 2 else slow):
+                    for _ in range(0 if layer % 2 else 6):
+                        big.fill_(layer)
+                    for t in src.layers[layer]:
+                        t.fill_(40 * step + layer)
+                    cli.record_event(layer)
+            m = ReqMeta()
+            m.dst_inst, m.dst_worker, m.reqid, m.dst_worker_info = "D|0|1", 0, "m%d" % step, srv.worker_info()
+            m.seen_tokens, m.new_tokens = 0, tokens
+            m.src_block_ids, m.dst_block_ids = [list(range(n))], [list(range(1, n + 1))]
+            cli.start_send_substep(step, 1, [m])
+            cli.flush_send_step()
+            assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+            torch.cuda.synchronize()
+            for layer in range(layers):
+                for rows in dst.rows(layer, 1, n):
+                    got = rows[:tokens]
+                    assert int(got.min()) == int(got.max()) == 40 * step + layer, (step, layer)
     finally:
         cli.drain()
         del cli
