@@ -1,6 +1,7 @@
 #include "core/completion.h"
 
 #include <pthread.h>
+#include <sys/prctl.h>
 
 #include <vector>
 
@@ -44,6 +45,10 @@ bool CompletionPoller::drain(std::chrono::milliseconds timeout) {
 
 void CompletionPoller::run() {
   pthread_setname_np(pthread_self(), "kvtcomplete");
+  // The kernel may round a sleep up by the thread's timer slack, 50 us by default: ten times the sleeps below.  A record that
+  // arrived behind the spin was then seen up to 55 us late (12 layers of hybrid pages, four requests of 1164 tokens: 207 us a
+  // step with the default, 168 with 1 us; 32 layers of 1111 tokens 158 and 116).
+  prctl(PR_SET_TIMERSLACK, 1000UL, 0, 0, 0);
   std::vector<Entry> ready;
   std::vector<PollResult> results;
   std::vector<const void*> blocked;

@@ -3,6 +3,7 @@ table helpers, KV specs of the model families."""
 import os
 import re
 import socket
+import time
 import zlib
 from pathlib import Path
 
@@ -211,6 +212,20 @@ def test_crash_trace_prints_native_frames_then_chains(ops):
     assert r.returncode == -11, (r.returncode, r.stderr[-500:])
     assert "kvtransfer crash trace: signal 11" in r.stderr and "end of trace" in r.stderr
     assert "(+0x" in r.stderr or "[0x" in r.stderr
+
+
+def test_the_completion_poller_sleeps_as_briefly_as_it_asks_to(ops):
+    """Its sleeps of 5 us last 55 with the default timer slack of 50 us."""
+    ops.completions_pending()          # the thread starts with the first use
+    slack = []
+    for _ in range(500):
+        for comm in Path("/proc/self/task").glob("*/comm"):
+            if comm.read_text().strip() == "kvtcomplete":
+                slack.append(int(Path("/proc", comm.parent.name, "timerslack_ns").read_text()))
+        if slack and slack[-1] <= 1000:
+            break
+        time.sleep(0.01)
+    assert slack and slack[-1] <= 1000
 
 
 def test_a_bounded_wait_of_a_warp_has_one_outcome_for_its_lanes():
