@@ -23,6 +23,7 @@
 #include "plan/planner.h"
 #include "topo/topology.h"
 #include "transport/channel.h"
+#include "transport/launch_run.h"
 #include "transport/peer_memory.h"
 
 namespace py = pybind11;
@@ -669,6 +670,8 @@ void bind_engine(py::module_& m) {
   m.def("fault_inject_arm", &fault_inject_arm);
   m.def("fault_inject_arm_drop_completion", &fault_inject_arm_drop_completion);
   m.def("fault_inject_arm_corrupt_check", &fault_inject_arm_corrupt_check);
+  m.def("layers_per_local_launch", &layers_per_local_launch, py::arg("remaining"), py::arg("bytes_per_layer"));
+  m.def("layers_per_remote_launch", &layers_per_remote_launch, py::arg("recorded"), py::arg("walk"));
   m.def("completions_pending", [] { return CompletionPoller::instance().pending(); });
   m.def("ipc_mappings_open", [] { return ipc_mappings_open(); },
         "Peer allocations this process has mapped through CUDA IPC handles right now.");

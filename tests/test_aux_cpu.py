@@ -242,3 +242,21 @@ def test_a_bounded_wait_of_a_warp_has_one_outcome_for_its_lanes():
         # what is left: the copy kernel's pipeline, which one lane drives
         assert rest.rindex("auto consume_one = [&]", 0, use.start()) > rest.rindex("__global__", 0, use.start())
     assert "if (lane == 0 && !failed) {" in rest and "while (!failed && stored < issued) consume_one();" in rest
+
+
+def test_layers_are_held_back_for_longer_launches_inside_one_gpu_only(ops):
+    local, remote = ops.layers_per_local_launch, ops.layers_per_remote_launch
+
+    def runs(layers, per):
+        out = []
+        while layers:
+            out.append(local(layers, per))
+            layers -= out[-1]
+        return out
+
+    assert runs(32, 32 << 20) == [4] * 6 + [4, 2, 1, 1]       # at most 128 MiB, then half of the rest
+    assert runs(32, 307200) == [16, 13, 3]                    # at least 4 MiB
+    assert runs(1, 1) == [1] and runs(3, 1 << 40) == [1, 1, 1] and runs(5, 0) == [5]
+    # another GPU: the link would idle meanwhile
+    assert [remote(n, False) for n in (1, 5, 32)] == [1, 1, 1]
+    assert [remote(n, True) for n in (1, 5, 32)] == [1, 5, 8]
