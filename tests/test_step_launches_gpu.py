@@ -274,3 +274,54 @@ def several_streams(shape, layers, tokens):
         cli.drain()
         del cli
         srv.stop()
+
+
+@pytest.mark.parametrize("host_gap_s", [0.0, 0.001])
+def test_one_step_towards_a_device_ordered_and_a_host_driven_destination(host_gap_s):
+    """The host-driven one wants to follow the layers one by one; the other lets the thread that waits for them sleep."""
+    layers, n = 12, 5
+    src = _Cache(CacheShape.FLASH, layers, n + 1)
+    dsts = [_Cache(CacheShape.FLASH, layers, n + 1) for _ in range(2)]
+    protos = [PT.NVLINK, PT.SHM]
+    srvs = [KVTransferServer("D%d|0|1" % i, 1, 0, 0, *(d.args[:4] + ([p],)), **d.kw) for i, (d, p) in enumerate(zip(dsts, protos))]
+    cli = KVTransferClient("P|0|1", 1, 0, 0, *(src.args[:4] + (protos,)), **src.kw)
+    try:
+        fwd = torch.cuda.Stream()
+        big = torch.empty(1 << 27, dtype=torch.uint8, device=DEV)
+
+        def submit(i, step):
+            cli.submit_req_send2("D%d|0|1" % i, 0, "r%d.%d" % (i, step), 0, n * BLOCK, True, list(range(n)), list(range(1, n + 1)),
+                                 srvs[i].worker_info(), stepid=step)
+
+        def meta(i, step):
+            m = ReqMeta()
+            m.dst_inst, m.dst_worker, m.reqid, m.dst_worker_info = "D%d|0|1" % i, 0, "s%d.%d" % (i, step), srvs[i].worker_info()
+            m.seen_tokens, m.new_tokens, m.src_block_ids, m.dst_block_ids = 0, n * BLOCK, [list(range(n))], [list(range(1, n + 1))]
+            return m
+
+        for step in range(1, 9):
+            late = step % 4                      # the host-driven destination: in the step from the start, or joins it later
+            submit(0, step)
+            if late == 0:
+                submit(1, step)
+            cli.start_send_step(step, 1)
+            for layer in range(layers):
+                with torch.cuda.stream(fwd):
+                    big.fill_(layer)
+                    src.layers[layer][0].fill_(16 * step + layer)
+                    cli.record_event(layer)
+                time.sleep(host_gap_s)
+                if layer == (0, 0, layers // 2, layers - 1)[late] and late:
+                    cli.start_send_substep(step, 1, [meta(1, step)])
+            cli.flush_send_step()
+            assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+            torch.cuda.synchronize()
+            for layer in range(layers):
+                for d in dsts:
+                    got = d.rows(layer, 1, n)[0]
+                    assert int(got.min()) == int(got.max()) == 16 * step + layer, (step, layer)
+    finally:
+        cli.drain()
+        del cli
+        for s in srvs:
+            s.stop()

@@ -9,7 +9,7 @@ import torch
 
 from llumnix_kv_b200.ops.layouts import AttnLayout, CacheShape
 from llumnix_kv_b200.ops.p2d_attn import (MODE_BF16_TO_MXFP8, MODE_COPY, MODE_MXFP8_TO_BF16, AttnTransfer, HeadMap, ReqChunk,
-                                          reference_transfer)
+                                          mx_quantize_reference, reference_transfer)
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -91,6 +91,40 @@ def test_quantiser_keeps_zero_groups_and_extremes():
         v[..., 65] = big
 
     _check(a, b, chunks, HeadMap(0, 0, 2), MODE_BF16_TO_MXFP8, prepare=prep)
+
+
+@pytest.mark.parametrize("dst_remote", [False, True])      # True: the staged form, whose stores this GPU takes as well
+@pytest.mark.parametrize("heads", [1, 8])                   # a warp a tile, four warps a tile
+def test_quantiser_with_infinities_and_nan(heads, dst_remote):
+    """A NaN does not count for its group's scale and keeps a NaN code; a group with an infinity takes the largest scale, 2^127,
+    whose reciprocal is zero in the kernel: NaN for the infinity and zero for the rest."""
+    pool, chunks = _chunks(random.Random(5), 16, [(0, 37)])
+    a = AttnLayout(CacheShape.FLASH, pool, 16, heads, 128, 2)
+    b = AttnLayout(CacheShape.FLASHINFER, pool, 16, heads, 128, 1, mx_scaled=True)
+    inf, nan = float("inf"), float("nan")
+    src, dst = _alloc(a, 1, 0), torch.zeros(b.layer_bytes, dtype=torch.uint8, device=DEV)
+    v = a.view(src, torch.bfloat16)
+    v[..., 0], v[..., 31] = nan, -nan           # both halves of a group: two lanes of the kernel
+    v[..., 32:64] = nan
+    v[..., 70] = inf
+    v[..., 90], v[..., 91] = nan, -inf
+    v[..., 96:128][..., ::2] = nan              # every other value
+    x = AttnTransfer(a, b, [src.data_ptr()], [dst.data_ptr()], DEV, head_map=HeadMap(0, 0, heads), mode=MODE_BF16_TO_MXFP8,
+                     dst_remote=dst_remote)
+    x.launch(x.plan(chunks))
+    torch.cuda.synchronize()
+    assert x.check_status() == (0, 0)
+    f = v.float().cpu()
+    q, e = b.view(dst, torch.uint8).cpu(), b.scale_view(dst).cpu()
+    c = chunks[0]
+    for t in range(37):
+        row = f[c.src_blocks[t // 16], :, t % 16]
+        want_q, want_e = mx_quantize_reference(torch.where(row.isnan(), torch.zeros(()), row))
+        got_q, got_e = q[c.dst_blocks[t // 16], :, t % 16], e[c.dst_blocks[t // 16], :, t % 16]
+        assert torch.equal(got_e, want_e)
+        is_nan = row.isnan() | row.isinf()
+        assert bool(((got_q & 0x7F) == 0x7F)[is_nan].all())
+        assert torch.equal(got_q[~is_nan], want_q[~is_nan])
 
 
 PAIRS = [(CacheShape.FLASH, CacheShape.FLASHINFER), (CacheShape.FLASHINFER, CacheShape.FLASH), (CacheShape.FLASH, CacheShape.FLASH),
