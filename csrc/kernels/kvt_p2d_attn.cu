@@ -1256,20 +1256,24 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
   int resident = grid;   // CTAs that are on the GPU together
   if (tma && grid_ctas <= 0 && a.dst_remote == 0 && tile_bytes != 0) {
     // Inside one GPU: as many CTAs per SM as have two tiles each in 200 KiB, 4 to 12.  One thread drives a CTA's tiles, so
-    // small ones want more CTAs: 500 tiles a layer of 4 KiB (1 head, 32 layers, 66 MB) 32.7 us with 4 or 6 a SM, 25 to 28 with
-    // 12 or 16; 80 layers 168 -> 142; 8 KiB tiles 189 -> 184.  32 KiB tiles keep 4: a lone launch of 291 MB takes
-    // 63.5 us so and 58.4 with 6, but one-layer launches of 1024 tiles overlapping on 8 streams 3172 and 2966 GB/s.
+    // small ones want more CTAs: 4 KiB tiles (1 head), 1024 a layer, 32 layers 64 us with 12 a SM, 85 with 6, 99 with 4; 8 KiB
+    // tiles, 16384 in all, 59 / 65 / 78.  Tiles of 32 KiB have one stage each at 4 to 6 a SM, so nothing but the other CTAs of
+    // the SM covers a CTA's wait.  They keep 4: one launch of 2048 or 5120 tiles takes 33.8 and 65.5 us with 4, 31.8 and 65.5
+    // with 6, but one-layer launches of 1024 tiles overlapping on 8 streams move 3172 and 2966 GB/s.
     const int per_sm = (int)std::min(12u, std::max(4u, kSmemBudget / 2u / tile_bytes));
     grid = resident = per_sm * sms;
-    // A long launch: CTAs of 128 KiB of tiles, handed to the SMs as they become free.  With a fixed share for each the
-    // slowest one ends the launch: 32 layers of 8192 tokens and 8 heads (1 GiB) took 361 us so and 341 with 3 to 4 tiles a
-    // CTA (343 with 7, 349 with 14); at 4 heads and 191 tiles a layer 77 us both ways, and 83 with one tile a CTA.
-    // Over NVLink the link bounds either.
+    // A long launch: CTAs of 128 KiB of tiles, handed to the SMs as they become free.  With a fixed share for each the slowest
+    // one ends the launch: 32 layers of 8192 tokens and 8 heads (32768 tiles, 1 GiB) take 339 us dealt out and 369 to 375 with
+    // a fixed share at 6 or 4 a SM, 12288 tiles 140 and 150.  Long means one and a half times the CTAs that run together (6 a SM
+    // at least): below that a mostly empty second wave costs more than it evens out.  us dealt out / fixed share: 4096 tiles
+    // (1.15 waves) 60 / 56, 5120 (1.44) 66 / 66, 5500 (1.55) 70 / 72, 6656 (1.87) 79 / 84; 16 KiB tiles (4 heads) 7168 (1.01) 57 /
+    // 49, 9216 (1.30) 64 / 60, 11000 (1.55) 70 / 70, 13312 (1.87) 81 / 83.  Over NVLink the link bounds either.
     const uint64_t tiles = tile_bytes < (128u << 10) ? (128u << 10) / tile_bytes : 1u;
     const uint64_t want = (total + tiles - 1) / tiles;
-    if (want > (uint64_t)grid) {
+    const int together = std::max(grid, 6 * sms);
+    if (want > (uint64_t)together + (uint64_t)together / 2u) {
       grid = (int)(want < (1u << 30) ? want : (1u << 30));
-      resident = std::max(resident, std::min(grid, 6 * sms));
+      resident = together;
     }
     if (threads <= 0) threads = 64;      // the second warp zeroes tails; 12 CTAs of 128 threads would not fit the registers
   }
