@@ -17,7 +17,8 @@
 // the destination layout, so the NHD<->HND permutation is done by the copy engine and the SM
 // issues two instructions per 8-32 KiB.  A ragged edge (a chunk that starts or ends inside a
 // block) is loaded as a whole tile and leaves as one untiled bulk store per contiguous run of
-// its own slots.  The fp8 paths and layouts TMA cannot describe run on a vector SIMT path.  TMA loads never use cluster multicast.
+// its own slots.  fp8 pages inside one GPU are expanded by a kernel of their own, fed by untiled bulk copies; the quantiser,
+// other expansions and layouts TMA cannot describe run on a vector SIMT path.  TMA loads never use cluster multicast.
 //
 // Every wait is bounded; on a bad block id or a timeout the kernel records a status word and
 // skips the access instead of faulting.
@@ -587,11 +588,11 @@ __device__ __forceinline__ void simt_zero_tail(const KvtAttnLaunch& p, const Til
   }
 }
 
-// Who owns a tile.  GROUP = 1: a warp (many tiles in flight per SM, nobody waits at tile boundaries;
-// best for long launches into device memory).  GROUP = 4: four warps share a tile, so that a
-// launch with few tiles still spreads over every SM and a whole tile is in flight at once (short
-// launches: one layer of a request).  GROUP = 0: the whole CTA (longer contiguous write runs, which
-// is what a PCIe destination prefers).  The owners of a CTA take consecutive tiles and the launcher
+// Who owns a tile.  GROUP = 1: a warp (many tiles in flight per SM, nobody waits at tile boundaries).
+// GROUP = 4: four warps share a tile, so that more of it is in flight at once, which tiles of 16 KiB
+// and more of the local quantiser gain by, in launches of any length (the figures are in launch_impl).
+// GROUP = 0: the whole CTA (longer contiguous write runs, which is what a PCIe destination prefers).
+// The owners of a CTA take consecutive tiles and the launcher
 // sizes the grid to the tiles, so that every resident CTA is full of busy warps: a CTA keeps its
 // registers until its last warp exits, and half-empty CTAs of one launch would keep the CTAs of
 // launches on other streams off the SM.
@@ -846,8 +847,11 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
 // Block-scaled fp8 -> bf16 inside one GPU is bound by HBM, and by how the tiles are read: a warp that walks a tile with
 // its own loads has 2 KiB of it in flight and comes back to the same DRAM pages many times.  Here warp 0 of a CTA walks the
 // block tables and brings each tile's rows and scale bytes into shared memory with untiled bulk copies, one per run that
-// the source holds contiguously, a tile ahead; the other warps convert from shared memory and store straight into the
-// destination.  Tiles pass through a ring of stages with a full and an empty mbarrier each.  Measured (HND fp8 -> NHD bf16,
+// the source holds contiguously; the other warps convert from shared memory and store straight into the destination.  Tiles
+// pass through a ring of as many stages as fit a sixth of an SM's shared memory, four at most, with a full and an empty mbarrier
+// each: tiles of up to 16 KiB of codes have one or more brought ahead of the one being converted.  Larger ones have a stage
+// alone, and the SM's other CTAs cover the wait for it: 16 heads (32 KiB), 16 layers of 2 x 3000 tokens, 596 MB, 106 us
+// against 174 with a warp per tile and 146 with four; one layer of 300 tokens 12, 60 and 22.  Measured (HND fp8 -> NHD bf16,
 // 8 heads, 32 layers of 3 x ~1334 tokens, 795 MB read and written): 197 us with a warp per tile, 178 with four, 170 with
 // eight, 144 this way (5.5 TB/s); one layer of 300 tokens 34 -> 11 us.  The other direction does not gain (the quantiser's
 // arithmetic fills the same warps: 174 against 158 us at 2 heads, 304 against 283 at 8) and stays with its own loads.
@@ -1093,15 +1097,16 @@ bool quant_staged(const KvtAttnLaunch& a) {
   return stage_env > 0 || (stage_env < 0 && a.dst_remote != 0);
 }
 
-// The expansion kernel serves what leaves the way of reading open (simt_tile 0), in tiles of at least 4 KiB of codes (with
-// 2 KiB, one head, the hand-over of a tile costs more than its reading: 32 layers of 6000 tokens 51 us against 43) of which
-// kConvCtas fit an SM; for the rest it says cudaErrorNotSupported and the SIMT kernel serves it.
-cudaError_t launch_expand(const KvtAttnLaunch& a, int grid_ctas, int sms, uint64_t total, cudaStream_t stream) {
+// The expansion kernel serves what leaves the way of reading open (simt_tile 0, no threads asked for: its CTAs have one size),
+// in tiles of at least 4 KiB of codes (with 2 KiB, one head, the hand-over of a tile costs more than its reading: 32 layers of
+// 6000 tokens 51 us against 43) of which kConvCtas fit an SM; for the rest it says cudaErrorNotSupported and the SIMT kernel
+// serves it.
+cudaError_t launch_expand(const KvtAttnLaunch& a, int grid_ctas, int threads_asked, int sms, uint64_t total, cudaStream_t stream) {
   const uint64_t rows = (uint64_t)a.n_heads * a.tile_tokens;
   const uint64_t tile_bytes = (rows * a.src.head_bytes + 127u) & ~127ull;
   const uint64_t stage_bytes = tile_bytes + ((rows * (a.src.head_bytes >> 5) + 127u) & ~127ull);
   const uint64_t budget = kSmemBudget / kConvCtas;
-  if (simt_choice(a) != 0 || a.dst_remote != 0 || tile_bytes < 4096u || stage_bytes > budget) return cudaErrorNotSupported;
+  if (threads_asked > 0 || simt_choice(a) != 0 || a.dst_remote != 0 || tile_bytes < 4096u || stage_bytes > budget) return cudaErrorNotSupported;
   uint64_t stages = budget / stage_bytes;
   if (stages > (uint64_t)kConvStages) stages = kConvStages;
   uint64_t grid = (uint64_t)grid_ctas;
@@ -1247,6 +1252,7 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (dev >= 0 && dev < kMaxDevices) sm_cache[dev].store(sms, std::memory_order_relaxed);
   }
+  const int threads_asked = threads;
   // Default: four CTAs per SM.  Many small CTAs, each with one tile in flight, measured faster
   // than one deep software pipeline per SM, and they let launches on different streams share SMs.
   int grid = grid_ctas > 0 ? grid_ctas : 4 * sms;
@@ -1310,7 +1316,7 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
     case KVT_MODE_BF16_TO_MXFP8:
       return (int)launch_impl<KVT_MODE_BF16_TO_MXFP8, false>(a, grid, threads, 0, 0, 0, stream);
     default:
-      if ((expand = launch_expand(a, grid_ctas, sms, total, stream)) != cudaErrorNotSupported) return (int)expand;
+      if ((expand = launch_expand(a, grid_ctas, threads_asked, sms, total, stream)) != cudaErrorNotSupported) return (int)expand;
       return (int)launch_impl<KVT_MODE_MXFP8_TO_BF16, false>(a, grid, threads, 0, 0, 0, stream);
   }
 }
