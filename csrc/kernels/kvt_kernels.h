@@ -109,8 +109,9 @@ typedef struct KvtAttnLaunch {
 uint32_t kvt_req_tiles(uint32_t seen, uint32_t new_tokens, uint32_t tile_tokens, uint32_t flags,
                        uint32_t dst_ntpb);
 
-// Launch the fused transfer kernel.  grid_ctas <= 0 picks one CTA per SM.  use_tma != 0 moves
-// full tiles with cp.async.bulk.tensor (needs src_maps/dst_maps and KVT_MODE_COPY).
+// Launch the fused transfer kernel.  grid_ctas <= 0 and threads <= 0: the launcher's choice.  use_tma != 0 loads tiles with
+// cp.async.bulk.tensor (needs src_maps/dst_maps and KVT_MODE_COPY): a full one leaves the same way or as one bulk store, a
+// partly filled one as a bulk store per contiguous run of its own slots.
 // Returns a cudaError_t value.
 int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int threads, int use_tma,
                         void* stream);

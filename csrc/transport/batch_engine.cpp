@@ -199,6 +199,11 @@ int BatchEngine::grid() const {
   return std::max(1, static_cast<int>(4 * kvt_sm_count(cfg_.device) * env_kernel_copy_sm_usage()));
 }
 
+int BatchEngine::attn_grid() const {
+  const bool asked = cfg_.grid_ctas > 0 || env_kernel_copy_sm_usage() < 1.0;
+  return cfg_.one_gpu && !asked ? 0 : grid();
+}
+
 void BatchEngine::ensure_attn_arrays(const DeviceAttnParams& p) {
   const bool same_maps = attn_ready_ && memcmp(&map_src_, &p.src, sizeof(KvtLayout)) == 0 &&
                          memcmp(&map_dst_, &p.dst, sizeof(KvtLayout)) == 0 && map_heads_ == p.n_heads &&
@@ -273,7 +278,7 @@ void BatchEngine::launch_attn(const DeviceAttnParams& params, const PackedPlan& 
   a.dst_remote = cfg_.dst_remote ? 1u : 0u;
   a.tile_order = tile_order_;
   a.store_form = store_form_;
-  cuda_check(kvt_launch_p2d_attn(&a, cfg_.one_gpu && cfg_.grid_ctas <= 0 && env_kernel_copy_sm_usage() >= 1.0 ? 0 : grid(), 0, use_tma_ ? 1 : 0, stream), "kvt_launch_p2d_attn");
+  cuda_check(kvt_launch_p2d_attn(&a, attn_grid(), 0, use_tma_ ? 1 : 0, stream), "kvt_launch_p2d_attn");
 }
 
 void BatchEngine::ensure_walk_arrays() {

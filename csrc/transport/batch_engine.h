@@ -37,8 +37,8 @@ struct BatchEngineConfig {
   size_t plan_capacity = 2u << 20;   // bytes per slot
   bool stamps = false;               // GPU timer stamps around every batch (DeviceUs in the metrics)
   bool dst_remote = false;           // the destination is another GPU's memory (quantiser staging, see kvt_kernels.h)
-  bool one_gpu = false;              // both caches live on this GPU: launches take the kernel's own grid rule
-  int grid_ctas = 0;                 // 0: four CTAs per SM scaled by the SM-usage knob
+  bool one_gpu = false;              // both caches live on this GPU (a pull session's source and a push's remote destination do not)
+  int grid_ctas = 0;                 // 0: four CTAs per SM scaled by the SM-usage knob, or see attn_grid()
 };
 
 class BatchEngine {
@@ -139,6 +139,7 @@ class BatchEngine {
   void ensure_attn_arrays(const DeviceAttnParams& p);
   void ensure_walk_arrays();
   int grid() const;
+  int attn_grid() const;             // 0: the attention kernel's own rule, where both caches share the GPU and no knob says otherwise
 
   BatchEngineConfig cfg_;
   std::vector<std::vector<uint64_t>> src_ptrs_, dst_ptrs_;

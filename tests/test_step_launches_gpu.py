@@ -44,7 +44,7 @@ class _Cache:
 @pytest.mark.parametrize("shape", [CacheShape.FLASH, CacheShape.DPSK_V32_SPARSE_MLA])
 @pytest.mark.parametrize("layers, tokens", [(1, 16), (2, 1), (13, 75), (13, 3001), (33, 700)])
 def test_every_layer_carries_what_was_recorded(layers, tokens, shape, host_gap_s):
-    """75 tokens: 4 MiB hold every layer.  3001: a quarter of the rest per launch.  host_gap_s: a forward thread slower than the
+    """75 tokens: 4 MiB hold every layer.  3001: half of the rest per launch.  host_gap_s: a forward thread slower than the
     sender, so that it waits for layers; without it the layers are all recorded long before the GPU has produced them."""
     n = -(-tokens // BLOCK)
     src, dst = _Cache(shape, layers, 2 * n + 2), _Cache(shape, layers, 2 * n + 2)
