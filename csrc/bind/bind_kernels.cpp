@@ -4,6 +4,7 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <algorithm>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -21,47 +22,100 @@ static void check_cuda(int err, const char* what) {
   }
 }
 
-// Host-side packing of a step's requests into the compact device plan: an array of
-// KvtReqDesc followed by the uint32 block-id pool, in one buffer so that one copy uploads it.
-struct PackedPlan {
-  py::bytes blob;
-  uint32_t n_reqs;
-  uint32_t total_tiles;
-  uint64_t block_ids_offset;  // byte offset of the pool inside blob
+// Host-side packing of a step's requests into the compact device plan: an array of KvtReqDesc followed by the uint32
+// block-id pool, in one buffer, which one copy uploads or a launch carries.
+struct HostPlan {
+  std::string blob;
+  uint32_t n_reqs = 0;
+  uint32_t total_tiles = 0;
+  uint64_t pool_offset = 0;  // byte offset of the block ids inside blob
+};
+
+struct PlanPacker {
+  const uint32_t tile_tokens, dst_ntpb;
+  std::vector<KvtReqDesc> descs;
+  std::vector<uint32_t> pool;
+  uint32_t tiles = 0;
+
+  // One request: the callables append its block ids of a side to the pool.
+  template <typename Src, typename Dst>
+  void add(Src&& src_ids, Dst&& dst_ids, uint32_t seen, uint32_t new_tokens, uint32_t flags) {
+    KvtReqDesc d{};
+    d.src_blk_off = static_cast<uint32_t>(pool.size());
+    src_ids(pool);
+    d.dst_blk_off = static_cast<uint32_t>(pool.size());
+    dst_ids(pool);
+    d.n_src_blocks = d.dst_blk_off - d.src_blk_off;
+    d.n_dst_blocks = static_cast<uint32_t>(pool.size()) - d.dst_blk_off;
+    d.seen_tokens = seen;
+    d.new_tokens = new_tokens;
+    d.flags = flags;
+    d.first_tile = tiles;
+    const uint32_t n = kvt_req_tiles(d.seen_tokens, d.new_tokens, tile_tokens, d.flags, dst_ntpb);
+    if (n == 0) return;
+    tiles += n;
+    descs.push_back(d);
+  }
+  HostPlan finish() const {
+    HostPlan out;
+    out.n_reqs = static_cast<uint32_t>(descs.size());
+    out.total_tiles = tiles;
+    out.pool_offset = descs.size() * sizeof(KvtReqDesc);
+    out.blob.resize(out.pool_offset + pool.size() * sizeof(uint32_t));
+    if (!descs.empty()) std::memcpy(out.blob.data(), descs.data(), out.pool_offset);
+    if (!pool.empty()) std::memcpy(out.blob.data() + out.pool_offset, pool.data(), pool.size() * sizeof(uint32_t));
+    return out;
+  }
 };
 
 static py::tuple pack_plan(const std::vector<std::tuple<std::vector<uint32_t>, std::vector<uint32_t>, uint32_t,
                                                         uint32_t, uint32_t>>& reqs,
                            uint32_t tile_tokens, uint32_t dst_ntpb) {
-  std::vector<KvtReqDesc> descs;
-  std::vector<uint32_t> pool;
-  descs.reserve(reqs.size());
-  uint32_t tiles = 0;
-  for (const auto& r : reqs) {
-    const auto& sb = std::get<0>(r);
-    const auto& db = std::get<1>(r);
-    KvtReqDesc d{};
-    d.src_blk_off = static_cast<uint32_t>(pool.size());
-    pool.insert(pool.end(), sb.begin(), sb.end());
-    d.dst_blk_off = static_cast<uint32_t>(pool.size());
-    pool.insert(pool.end(), db.begin(), db.end());
-    d.n_src_blocks = static_cast<uint32_t>(sb.size());
-    d.n_dst_blocks = static_cast<uint32_t>(db.size());
-    d.seen_tokens = std::get<2>(r);
-    d.new_tokens = std::get<3>(r);
-    d.flags = std::get<4>(r);
-    d.first_tile = tiles;
-    const uint32_t n = kvt_req_tiles(d.seen_tokens, d.new_tokens, tile_tokens, d.flags, dst_ntpb);
-    if (n == 0) continue;
-    tiles += n;
-    descs.push_back(d);
+  PlanPacker pk{tile_tokens, dst_ntpb, {}, {}};
+  auto ids = [](const std::vector<uint32_t>& v) {
+    return [&v](std::vector<uint32_t>& pool) { pool.insert(pool.end(), v.begin(), v.end()); };
+  };
+  for (const auto& r : reqs) pk.add(ids(std::get<0>(r)), ids(std::get<1>(r)), std::get<2>(r), std::get<3>(r), std::get<4>(r));
+  const HostPlan p = pk.finish();
+  return py::make_tuple(py::bytes(p.blob), p.n_reqs, p.total_tiles, p.pool_offset);
+}
+
+// An unsigned 32-bit number: a plain int is read directly, anything else through `convert` (PyNumber_Index or PyNumber_Long).
+static uint32_t as_u32(PyObject* o, PyObject* (*convert)(PyObject*)) {
+  if (!PyLong_CheckExact(o)) {
+    const py::object whole = py::reinterpret_steal<py::object>(convert(o));
+    if (!whole) throw py::error_already_set();
+    if (PyLong_CheckExact(whole.ptr())) return as_u32(whole.ptr(), convert);
+    throw py::type_error("kvt_pack_chunks: not a whole number");
   }
-  const size_t desc_bytes = descs.size() * sizeof(KvtReqDesc);
-  std::string blob(desc_bytes + pool.size() * sizeof(uint32_t), '\0');
-  if (desc_bytes) std::memcpy(blob.data(), descs.data(), desc_bytes);
-  if (!pool.empty()) std::memcpy(blob.data() + desc_bytes, pool.data(), pool.size() * sizeof(uint32_t));
-  return py::make_tuple(py::bytes(blob), static_cast<uint32_t>(descs.size()), tiles,
-                        static_cast<uint64_t>(desc_bytes));
+  const unsigned long v = PyLong_AsUnsignedLong(o);
+  if (v == static_cast<unsigned long>(-1) && PyErr_Occurred()) throw py::error_already_set();
+  if (v > 0xffffffffull) throw py::value_error("kvt_pack_chunks: number beyond 32 bits");
+  return static_cast<uint32_t>(v);
+}
+
+// The same from chunk objects (src_blocks, dst_blocks, seen_tokens, new_tokens, pad_tail) without a Python list per table.
+static HostPlan pack_chunks(const py::iterable& chunks, uint32_t tile_tokens, uint32_t dst_ntpb) {
+  PlanPacker pk{tile_tokens, dst_ntpb, {}, {}};
+  for (const py::handle c : chunks) {
+    auto ids = [&c](const char* name) {
+      return [&c, name](std::vector<uint32_t>& pool) {
+        const py::object table = c.attr(name);
+        const py::object seq = py::reinterpret_steal<py::object>(PySequence_Fast(table.ptr(), "block ids are a sequence"));
+        if (!seq) throw py::error_already_set();
+        for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq.ptr()); ++i) {
+          const py::object id = py::reinterpret_borrow<py::object>(PySequence_Fast_GET_ITEM(seq.ptr(), i));
+          pool.push_back(as_u32(id.ptr(), &PyNumber_Index));
+        }
+      };
+    };
+    const py::object seen = c.attr("seen_tokens"), fresh = c.attr("new_tokens"), pad = c.attr("pad_tail");
+    const int padded = PyObject_IsTrue(pad.ptr());
+    if (padded < 0) throw py::error_already_set();
+    pk.add(ids("src_blocks"), ids("dst_blocks"), as_u32(seen.ptr(), &PyNumber_Long), as_u32(fresh.ptr(), &PyNumber_Long),
+           padded != 0 ? KVT_REQ_PAD_TAIL : 0u);
+  }
+  return pk.finish();
 }
 
 void bind_kernels(py::module_& m) {
@@ -105,6 +159,20 @@ void bind_kernels(py::module_& m) {
   m.attr("KVT_SEG_RULE_BYTES") = static_cast<int>(sizeof(KvtSegRule));
   m.attr("KVT_TENSOR_MAP_BYTES") = 128;
 
+  m.attr("KVT_PLAN_IN_LAUNCH") = static_cast<int>(KVT_PLAN_IN_LAUNCH);
+
+  py::class_<HostPlan>(m, "HostPlan")
+      .def_readonly("n_reqs", &HostPlan::n_reqs)
+      .def_readonly("total_tiles", &HostPlan::total_tiles)
+      .def_readonly("pool_offset", &HostPlan::pool_offset)
+      .def_property_readonly("nbytes", [](const HostPlan& p) { return p.blob.size(); })
+      .def_property_readonly("blob", [](const HostPlan& p) { return py::bytes(p.blob); })
+      .def("copy_to_device", [](const HostPlan& p, uint64_t dst) {
+        if (!p.blob.empty()) check_cuda(kvt_copy_now(dst, p.blob.data(), p.blob.size()), "kvt_copy_now");
+      }, "The plan at a device address, complete on return and outside of any capture.");
+  m.def("kvt_pack_chunks", &pack_chunks, py::arg("chunks"), py::arg("tile_tokens"), py::arg("dst_ntpb"));
+  m.def("kvt_stream_capturing", [](uint64_t stream) { return kvt_stream_capturing(reinterpret_cast<void*>(stream)) != 0; });
+
   m.def("kvt_req_tiles", &kvt_req_tiles);
   m.def("kvt_pack_plan", &pack_plan, py::arg("reqs"), py::arg("tile_tokens"), py::arg("dst_ntpb"),
         "Pack [(src_blocks, dst_blocks, seen, new, flags)] into (blob, n_reqs, total_tiles, pool_offset).");
@@ -129,8 +197,13 @@ void bind_kernels(py::module_& m) {
          uint32_t total_tiles, uint64_t block_ids, uint32_t tile_tokens, uint32_t src_head0, uint32_t dst_head0,
          uint32_t n_heads, uint32_t mode, uint64_t status, uint64_t done_counter, uint64_t flag,
          uint64_t flag_value, int grid, int threads, int use_tma, uint64_t stream, uint32_t simt_tile,
-         uint32_t dst_remote, uint32_t tile_order, uint32_t store_form, uint32_t tma_stages, uint32_t cache_hint) {
+         uint32_t dst_remote, uint32_t tile_order, uint32_t store_form, uint32_t tma_stages, uint32_t cache_hint,
+         const HostPlan* plan) {
         KvtAttnLaunch a{};
+        if (plan != nullptr) {
+          a.plan = plan->blob.data();
+          a.plan_bytes = static_cast<uint32_t>(std::min<size_t>(plan->blob.size(), 0xffffffffu));
+        }
         a.simt_tile = simt_tile;
         a.dst_remote = dst_remote;
         a.tile_order = tile_order;
@@ -167,7 +240,7 @@ void bind_kernels(py::module_& m) {
       py::arg("dst_head0"), py::arg("n_heads"), py::arg("mode"), py::arg("status"), py::arg("done_counter"),
       py::arg("flag"), py::arg("flag_value"), py::arg("grid"), py::arg("threads"), py::arg("use_tma"),
       py::arg("stream"), py::arg("simt_tile") = 0, py::arg("dst_remote") = 0, py::arg("tile_order") = 0,
-      py::arg("store_form") = 0, py::arg("tma_stages") = 0, py::arg("cache_hint") = 0);
+      py::arg("store_form") = 0, py::arg("tma_stages") = 0, py::arg("cache_hint") = 0, py::arg("plan") = nullptr);
 
   m.def(
       "kvt_launch_p2d_state",

@@ -67,6 +67,10 @@ enum KvtStatus {
   KVT_ERR_FLAG_TIMEOUT = 4,    // a bounded wait on a completion flag ran out
 };
 
+// Bytes of a plan ([KvtReqDesc x n_reqs][block ids]) that a launch can carry in its own parameters, beside the rest of them below
+// the 4 KiB of parameters that every launch may have: 444 blocks a side of one request.
+#define KVT_PLAN_IN_LAUNCH 3584u
+
 typedef struct KvtAttnLaunch {
   const uint64_t* src_layers;  // device array, one base address per layer (local memory)
   const uint64_t* dst_layers;  // device array, one base address per layer (local / peer / host-mapped)
@@ -103,6 +107,8 @@ typedef struct KvtAttnLaunch {
                                // run of the destination, which then crosses NVLink as one linear write
   uint32_t tma_stages;         // cap of the per-CTA pipeline depth (0: as many as shared memory allows, at most 8)
   uint32_t cache_hint;         // 1: L2 evict_first policy on the tile loads and stores (streamed once)
+  const void* plan;            // host memory or NULL: the whole plan, at most KVT_PLAN_IN_LAUNCH bytes, read before the call
+  uint32_t plan_bytes;         // returns; `reqs` and `block_ids` are not used then, and nothing has to be uploaded
 } KvtAttnLaunch;
 
 // Tile count of one request for a given tile size (host helper, also used by tests).
@@ -425,6 +431,10 @@ int kvt_host_alloc_mapped(uint64_t bytes, uint64_t* host_ptr, uint64_t* dev_ptr)
 int kvt_host_free(uint64_t host_ptr);
 int kvt_host_register(uint64_t host_ptr, uint64_t bytes, uint64_t* dev_ptr);
 int kvt_host_unregister(uint64_t host_ptr);
+// 1: the stream is being captured into a graph.
+int kvt_stream_capturing(void* stream);
+// host -> device copy that is complete on return and stays out of any capture that is going on.
+int kvt_copy_now(uint64_t dst, const void* src, uint64_t bytes);
 int kvt_sm_count(int dev);
 // Copy-engine copies by raw address (device, peer-mapped or pinned host memory on either side): one
 // cudaMemcpyAsync, or one per {src_off, dst_off, len} triple of a host array.  They are the library

@@ -492,6 +492,32 @@ extern "C" int kvt_host_unregister(uint64_t host_ptr) {
   return (int)cudaHostUnregister(reinterpret_cast<void*>(host_ptr));
 }
 
+extern "C" int kvt_stream_capturing(void* stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(stream), &st) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return st == cudaStreamCaptureStatusNone ? 0 : 1;
+}
+
+extern "C" int kvt_copy_now(uint64_t dst, const void* src, uint64_t bytes) {
+  // relaxed for this thread: calls on a stream that nobody captures are then allowed while another stream is being captured
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return (int)e;
+  cudaStream_t s = nullptr;
+  e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) {
+    e = cudaMemcpyAsync(reinterpret_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice, s);
+    const cudaError_t w = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = w;
+    cudaStreamDestroy(s);
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return (int)e;
+}
+
 // ---- copy-engine paths: the in-run bandwidth ceilings and the library baseline of the benchmark ----
 extern "C" int kvt_memcpy_async(uint64_t dst, uint64_t src, uint64_t bytes, void* stream) {
   return (int)cudaMemcpyAsync(reinterpret_cast<void*>(dst), reinterpret_cast<const void*>(src), bytes, cudaMemcpyDefault,

@@ -24,6 +24,7 @@
 // skips the access instead of faulting.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -31,6 +32,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include "kvt_kernels.h"
 
@@ -61,20 +63,53 @@ __device__ __forceinline__ void set_status(uint32_t* status, uint32_t code, uint
   }
 }
 
+// Where the plan is.  A short one travels in the launch's parameters (IN_LAUNCH): its upload would be a copy in front of the
+// kernel and, from Python, a pinned buffer and a device tensor.  us a pass with an uploaded plan / this way, packing included: one
+// layer of 333 tokens 33.1 / 8.9, fp8 -> bf16 of 32 layers of 4003 tokens 147 / 137, 24 blocks to host memory 1034 / 999.
+// The lanes read it by generic addresses, coalesced as from memory: an index into the parameter space would be served lane by lane.
+template <bool IN_LAUNCH>
+struct PlanParam {};
+template <>
+struct PlanParam<true> {
+  uint32_t words[KVT_PLAN_IN_LAUNCH / 4u];
+};
+template <bool IN_LAUNCH>
+struct PlanView {
+  const KvtReqDesc* reqs;
+  const uint32_t* block_ids;
+  __device__ __forceinline__ PlanView(const KvtAttnLaunch& p, const PlanParam<IN_LAUNCH>& param) {
+    if constexpr (IN_LAUNCH) {
+      uint64_t at = reinterpret_cast<uint64_t>(&param.words[0]);
+      asm volatile("" : "+l"(at));
+      reqs = reinterpret_cast<const KvtReqDesc*>(at);
+      block_ids = reinterpret_cast<const uint32_t*>(at + (uint64_t)p.n_reqs * sizeof(KvtReqDesc));
+    } else {
+      reqs = p.reqs;
+      block_ids = p.block_ids;
+    }
+  }
+  __device__ __forceinline__ uint32_t load(const uint32_t* w) const {
+    if constexpr (IN_LAUNCH) return *w;
+    else return __ldg(w);
+  }
+};
+
 // Largest r with reqs[r].first_tile <= t.
-__device__ __forceinline__ uint32_t find_req(const KvtReqDesc* __restrict__ reqs, uint32_t n, uint32_t t) {
+template <bool IN_LAUNCH>
+__device__ __forceinline__ uint32_t find_req(const PlanView<IN_LAUNCH>& plan, uint32_t n, uint32_t t) {
   uint32_t lo = 0, hi = n;
   while (hi - lo > 1) {
     uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(&reqs[mid].first_tile) <= t) lo = mid; else hi = mid;
+    if (plan.load(&plan.reqs[mid].first_tile) <= t) lo = mid; else hi = mid;
   }
   return lo;
 }
 
-__device__ __forceinline__ TileInfo decode_tile(const KvtAttnLaunch& p, uint32_t tile) {
+template <bool IN_LAUNCH>
+__device__ __forceinline__ TileInfo decode_tile(const KvtAttnLaunch& p, const PlanView<IN_LAUNCH>& plan, uint32_t tile) {
   TileInfo ti;
-  const uint32_t r = find_req(p.reqs, p.n_reqs, tile);
-  const KvtReqDesc rd = p.reqs[r];
+  const uint32_t r = find_req(plan, p.n_reqs, tile);
+  const KvtReqDesc rd = plan.reqs[r];
   const uint32_t tt = p.tile_tokens;
   const uint32_t local = tile - rd.first_tile;
   const uint32_t tok_lo = (rd.seen_tokens / tt + local) * tt;
@@ -101,14 +136,14 @@ __device__ __forceinline__ TileInfo decode_tile(const KvtAttnLaunch& p, uint32_t
     if (sbi >= rd.n_src_blocks) {
       ti.ok = false;
     } else {
-      ti.sblk = __ldg(&p.block_ids[rd.src_blk_off + sbi]);
+      ti.sblk = plan.load(&plan.block_ids[rd.src_blk_off + sbi]);
       if (ti.sblk >= p.src.num_blocks) ti.ok = false;
     }
   }
   if (dbi >= rd.n_dst_blocks) {
     ti.ok = false;
   } else {
-    ti.dblk = __ldg(&p.block_ids[rd.dst_blk_off + dbi]);
+    ti.dblk = plan.load(&plan.block_ids[rd.dst_blk_off + dbi]);
     if (ti.dblk >= p.dst.num_blocks) ti.ok = false;
   }
   return ti;
@@ -596,8 +631,8 @@ __device__ __forceinline__ void simt_zero_tail(const KvtAttnLaunch& p, const Til
 // sizes the grid to the tiles, so that every resident CTA is full of busy warps: a CTA keeps its
 // registers until its last warp exits, and half-empty CTAs of one launch would keep the CTAs of
 // launches on other streams off the SM.
-template <int MODE, bool USE_TMA, int GROUP>
-__device__ __forceinline__ void simt_pass(const KvtAttnLaunch& p, uint64_t total, uint32_t per_layer,
+template <int MODE, bool USE_TMA, int GROUP, bool IN_LAUNCH>
+__device__ __forceinline__ void simt_pass(const KvtAttnLaunch& p, const PlanView<IN_LAUNCH>& plan, uint64_t total, uint32_t per_layer,
                                           unsigned char* stage_base) {
   constexpr uint32_t kGroupThreads = GROUP > 0 ? 32u * GROUP : 0u;
   const uint32_t tid = GROUP > 0 ? (threadIdx.x % kGroupThreads) : threadIdx.x;
@@ -619,7 +654,7 @@ __device__ __forceinline__ void simt_pass(const KvtAttnLaunch& p, uint64_t total
     if (w < total) {
       uint32_t tile;
       split_work(p, w, total, per_layer, mine.layer, mine.kv, tile);
-      const TileInfo ti = decode_tile(p, tile);
+      const TileInfo ti = decode_tile(p, plan, tile);
       if (!ti.ok) {
         if (tid < 32u) set_status(p.status, KVT_ERR_BLOCK_RANGE, tile);
       } else {
@@ -693,11 +728,13 @@ __device__ __forceinline__ void publish_completion(const KvtAttnLaunch& p) {
 }
 
 // ---- the kernel ---------------------------------------------------------------------------
-template <int MODE, bool USE_TMA>
+template <int MODE, bool USE_TMA, bool IN_LAUNCH>
 __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_constant__ KvtAttnLaunch p,
                                                             const uint32_t n_stages, const uint32_t tile_bytes,
-                                                            const uint32_t warp_tiles) {
+                                                            const uint32_t warp_tiles,
+                                                            const __grid_constant__ PlanParam<IN_LAUNCH> plan_param) {
   extern __shared__ __align__(1024) unsigned char smem[];
+  const PlanView<IN_LAUNCH> plan(p, plan_param);
   const uint32_t n_layers = p.layer_end - p.layer_begin;
   const uint32_t per_layer = p.total_tiles * p.src.kv_count;
   const uint64_t total = (uint64_t)n_layers * per_layer;
@@ -764,7 +801,7 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
         if (w < total) {
           uint32_t tile;
           split_work(p, w, total, per_layer, layer, kv, tile);
-          ti = decode_tile(p, tile);
+          ti = decode_tile(p, plan, tile);
           mine = ti.ok && ti.copy_hi > ti.copy_lo;  // bad tiles are reported by the SIMT pass
         }
         const unsigned any = __ballot_sync(0xffffffffu, w < total);
@@ -833,11 +870,11 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
   // without TMA tiles a non-zero tile_bytes says that every warp owns a staging buffer of that size
   unsigned char* stage_base = (!USE_TMA && tile_bytes == kStagePerWarp) ? smem : nullptr;
   if (warp_tiles == 1u) {
-    simt_pass<MODE, USE_TMA, 1>(p, total, per_layer, stage_base);
+    simt_pass<MODE, USE_TMA, 1>(p, plan, total, per_layer, stage_base);
   } else if (warp_tiles == 4u) {
-    simt_pass<MODE, USE_TMA, 4>(p, total, per_layer, nullptr);
+    simt_pass<MODE, USE_TMA, 4>(p, plan, total, per_layer, nullptr);
   } else {
-    simt_pass<MODE, USE_TMA, 0>(p, total, per_layer, nullptr);
+    simt_pass<MODE, USE_TMA, 0>(p, plan, total, per_layer, nullptr);
   }
 
   publish_completion(p);
@@ -900,10 +937,13 @@ struct ConvRows {
   }
 };
 
+template <bool IN_LAUNCH>
 __global__ void __launch_bounds__(kConvThreads, kConvCtas) kvt_p2d_expand_kernel(const __grid_constant__ KvtAttnLaunch p,
                                                                                const uint32_t n_stages, const uint32_t tile_bytes,
-                                                                               const uint32_t stage_bytes) {
+                                                                               const uint32_t stage_bytes,
+                                                                               const __grid_constant__ PlanParam<IN_LAUNCH> plan_param) {
   extern __shared__ __align__(1024) unsigned char smem[];
+  const PlanView<IN_LAUNCH> plan(p, plan_param);
   __shared__ uint64_t full[kConvStages], empty[kConvStages];
   __shared__ ConvSlot slots[kConvStages];
   const uint32_t per_layer = p.total_tiles * p.src.kv_count;
@@ -941,7 +981,7 @@ __global__ void __launch_bounds__(kConvThreads, kConvCtas) kvt_p2d_expand_kernel
       if (w < total) {
         uint32_t tile;
         split_work(p, w, total, per_layer, mine.layer, mine.kv, tile);
-        const TileInfo ti = decode_tile(p, tile);
+        const TileInfo ti = decode_tile(p, plan, tile);
         if (ti.ok) work = mine.set(ti); else set_status(p.status, KVT_ERR_BLOCK_RANGE, tile);
       }
       for (unsigned todo = __ballot_sync(0xffffffffu, work); todo != 0u; todo &= todo - 1u) {
@@ -1097,6 +1137,14 @@ bool quant_staged(const KvtAttnLaunch& a) {
   return stage_env > 0 || (stage_env < 0 && a.dst_remote != 0);
 }
 
+// The plan as a parameter of the launch.
+template <bool IN_LAUNCH>
+PlanParam<IN_LAUNCH> plan_param(const KvtAttnLaunch& a) {
+  PlanParam<IN_LAUNCH> out;
+  if constexpr (IN_LAUNCH) memcpy(out.words, a.plan, a.plan_bytes);
+  return out;
+}
+
 // The expansion kernel serves what leaves the way of reading open (simt_tile 0, no threads asked for: its CTAs have one size),
 // in tiles of at least 4 KiB of codes (with 2 KiB, one head, the hand-over of a tile costs more than its reading: 32 layers of
 // 6000 tokens 51 us against 43) of which kConvCtas fit an SM; for the rest it says cudaErrorNotSupported and the SIMT kernel
@@ -1116,7 +1164,32 @@ cudaError_t launch_expand(const KvtAttnLaunch& a, int grid_ctas, int threads_ask
   }
   if (grid > total) grid = total;
   // at most kSmemBudget / kConvCtas bytes: below the 48 KiB that need no opt-in
-  kvt_p2d_expand_kernel<<<(int)grid, kConvThreads, stages * stage_bytes, stream>>>(a, (uint32_t)stages, (uint32_t)tile_bytes, (uint32_t)stage_bytes);
+  const auto go = [&](auto in_launch) {
+    constexpr bool kIn = decltype(in_launch)::value;
+    kvt_p2d_expand_kernel<kIn><<<(int)grid, kConvThreads, stages * stage_bytes, stream>>>(a, (uint32_t)stages, (uint32_t)tile_bytes,
+                                                                                         (uint32_t)stage_bytes, plan_param<kIn>(a));
+  };
+  if (a.plan != nullptr) go(std::true_type{}); else go(std::false_type{});
+  return cudaGetLastError();
+}
+
+template <int MODE, bool USE_TMA, bool IN_LAUNCH>
+cudaError_t launch_as(const KvtAttnLaunch& a, int grid, int threads, uint32_t stages, uint32_t tile_bytes, size_t smem,
+                      uint32_t warp_tiles, cudaStream_t stream) {
+  auto kern = kvt_p2d_attn_kernel<MODE, USE_TMA, IN_LAUNCH>;
+  if (smem > 48 * 1024) {
+    // the opt-in is per device and sticky: ask once per device (and again only for a larger size)
+    static std::atomic<size_t> granted[kMaxDevices];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::atomic<size_t>* slot = dev >= 0 && dev < kMaxDevices ? &granted[dev] : nullptr;
+    if (slot == nullptr || slot->load(std::memory_order_relaxed) < smem) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      if (slot != nullptr) slot->store(smem, std::memory_order_relaxed);
+    }
+  }
+  kern<<<grid, threads, smem, stream>>>(a, stages, tile_bytes, warp_tiles, plan_param<IN_LAUNCH>(a));
   return cudaGetLastError();
 }
 
@@ -1149,21 +1222,8 @@ cudaError_t launch_impl(const KvtAttnLaunch& a, int grid, int threads, uint32_t 
       smem = (size_t)warps * kStagePerWarp;
     }
   }
-  auto kern = kvt_p2d_attn_kernel<MODE, USE_TMA>;
-  if (smem > 48 * 1024) {
-    // the opt-in is per device and sticky: ask once per device (and again only for a larger size)
-    static std::atomic<size_t> granted[kMaxDevices];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::atomic<size_t>* slot = dev >= 0 && dev < kMaxDevices ? &granted[dev] : nullptr;
-    if (slot == nullptr || slot->load(std::memory_order_relaxed) < smem) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      if (slot != nullptr) slot->store(smem, std::memory_order_relaxed);
-    }
-  }
-  kern<<<grid, threads, smem, stream>>>(a, stages, tile_bytes, warp_tiles);
-  return cudaGetLastError();
+  return a.plan != nullptr ? launch_as<MODE, USE_TMA, true>(a, grid, threads, stages, tile_bytes, smem, warp_tiles, stream)
+                           : launch_as<MODE, USE_TMA, false>(a, grid, threads, stages, tile_bytes, smem, warp_tiles, stream);
 }
 
 }  // namespace
@@ -1230,6 +1290,8 @@ extern "C" int kvt_launch_p2d_attn(const KvtAttnLaunch* args, int grid_ctas, int
   const KvtAttnLaunch& a = *args;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (a.n_reqs == 0 || a.total_tiles == 0 || a.layer_end <= a.layer_begin) return (int)cudaSuccess;
+  if (a.plan != nullptr && (a.plan_bytes > KVT_PLAN_IN_LAUNCH || a.plan_bytes < (uint64_t)a.n_reqs * sizeof(KvtReqDesc)))
+    return (int)cudaErrorInvalidValue;
   if (a.tile_tokens == 0 || a.src.ntpb % a.tile_tokens != 0 || a.dst.ntpb % a.tile_tokens != 0)
     return (int)cudaErrorInvalidValue;
   if (a.src.kv_count != a.dst.kv_count || a.n_heads == 0) return (int)cudaErrorInvalidValue;

@@ -159,6 +159,7 @@ BatchEngine::SlotView BatchEngine::begin(size_t bytes) {
   {
     std::lock_guard<std::mutex> g(slot_mu_);
     sl.seq = ++next_seq_;
+    sl.in_launches = 0;
     sl.metrics.clear();
   }
   batch_slot_ = static_cast<int>(slot_rr_);
@@ -166,8 +167,10 @@ BatchEngine::SlotView BatchEngine::begin(size_t bytes) {
   return SlotView{sl.h_plan, sl.d_plan, sl.d_status, sl.seq};
 }
 
-void BatchEngine::upload(size_t bytes) {
+void BatchEngine::upload(size_t bytes, bool in_launches) {
   Slot& sl = cur();
+  sl.in_launches = in_launches && !cfg_.stamps && bytes <= KVT_PLAN_IN_LAUNCH ? static_cast<uint32_t>(bytes) : 0u;
+  if (sl.in_launches != 0) return;
   if (bytes != 0)
     cuda_check(cudaMemcpyAsync(sl.d_plan, sl.h_plan, bytes, cudaMemcpyHostToDevice, sl.stream), "cudaMemcpyAsync(plan)");
   if (cfg_.stamps) cuda_check(kvt_launch_stamp(reinterpret_cast<uint64_t*>(sl.d_status) + 1, sl.stream), "kvt_launch_stamp");
@@ -177,7 +180,7 @@ void BatchEngine::upload(size_t bytes) {
 DeviceStage& BatchEngine::stage(size_t i) {
   if (stage_used_.size() != stages_.size()) stage_used_.assign(stages_.size(), 0);
   if (!stage_used_[i]) {
-    stages_[i]->wait_event(cur().plan_event);
+    if (cur().in_launches == 0) stages_[i]->wait_event(cur().plan_event);
     stage_used_[i] = 1;
   }
   return *stages_[i];
@@ -265,6 +268,10 @@ void BatchEngine::launch_attn(const DeviceAttnParams& params, const PackedPlan& 
   a.dst = params.dst;
   a.layer_begin = static_cast<uint32_t>(lo);
   a.layer_end = static_cast<uint32_t>(hi);
+  if (sl.in_launches != 0) {
+    a.plan = sl.h_plan;
+    a.plan_bytes = sl.in_launches;
+  }
   a.reqs = reinterpret_cast<const KvtReqDesc*>(sl.d_plan);
   a.n_reqs = plan.n_reqs;
   a.total_tiles = plan.total_tiles;

@@ -62,7 +62,9 @@ class BatchEngine {
   BatchEngine(const BatchEngine&) = delete;
 
   SlotView begin(size_t bytes);
-  void upload(size_t bytes);
+  // `in_launches`: the batch is made of attention launches only, which carry a plan that is short enough themselves: nothing is
+  // uploaded then and the transfer streams have nothing to join.
+  void upload(size_t bytes, bool in_launches = false);
   SlotView current();
   bool in_batch() const { return batch_slot_ >= 0; }
   // Transfer stream `i` of the current batch (joined to the plan upload at first use).
@@ -115,6 +117,7 @@ class BatchEngine {
     KvtCompletion* h_rec{nullptr};
     KvtCompletion* d_rec{nullptr};
     uint64_t seq{0};
+    uint32_t in_launches{0};           // bytes of h_plan that the launches carry (0: the plan is uploaded)
     bool pending{false};
     std::string metrics;
   };

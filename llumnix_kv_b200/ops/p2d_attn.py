@@ -59,27 +59,45 @@ class HeadMap:
 
 
 class DevicePlan:
-    """A step's requests packed for the kernel and uploaded with one copy."""
+    """A step's requests packed for the kernel.
+
+    A short plan stays on the host and travels in the parameters of its launches, until somebody asks for its device
+    buffer (``dev``) or a launch is captured into a graph, whose replays read the buffer: from then on the launches read
+    it too, so that it can be overwritten in place.  A long one, or one with a ``pinned`` buffer to go through, is
+    uploaded with one copy at once."""
 
     def __init__(self, chunks: Sequence[ReqChunk], tile_tokens: int, dst_ntpb: int, device, stream=None,
                  pinned: Optional[torch.Tensor] = None):
         K = _ops()
-        blob, self.n_reqs, self.total_tiles, pool_off = K.kvt_pack_plan([c.as_tuple() for c in chunks],
-                                                                       tile_tokens, dst_ntpb)
-        self.nbytes = len(blob)
-        self.pool_offset = pool_off
+        self._host = host = K.kvt_pack_chunks(chunks, tile_tokens, dst_ntpb)
+        self.n_reqs, self.total_tiles, self.pool_offset, self.nbytes = host.n_reqs, host.total_tiles, host.pool_offset, host.nbytes
+        self.pinned, self.device = pinned, device
+        self._dev: Optional[torch.Tensor] = None
+        if pinned is None and self.nbytes <= K.KVT_PLAN_IN_LAUNCH:
+            return
         n = max(self.nbytes, 16)
         if pinned is None or pinned.numel() < n:
-            pinned = torch.empty(n, dtype=torch.uint8, pin_memory=torch.cuda.is_available())
-        self.pinned = pinned
+            self.pinned = pinned = torch.empty(n, dtype=torch.uint8, pin_memory=torch.cuda.is_available())
         if self.nbytes:
-            pinned[: self.nbytes].copy_(torch.frombuffer(bytearray(blob), dtype=torch.uint8))
-        self.dev = torch.empty(n, dtype=torch.uint8, device=device)
+            pinned[: self.nbytes].copy_(torch.frombuffer(bytearray(host.blob), dtype=torch.uint8))
+        self._dev = torch.empty(n, dtype=torch.uint8, device=device)
         if stream is None:
-            self.dev.copy_(pinned[:n], non_blocking=True)
+            self._dev.copy_(pinned[:n], non_blocking=True)
         else:
             with torch.cuda.stream(stream):
-                self.dev.copy_(pinned[:n], non_blocking=True)
+                self._dev.copy_(pinned[:n], non_blocking=True)
+
+    @property
+    def dev(self) -> torch.Tensor:
+        if self._dev is None:
+            dev = torch.empty(max(self.nbytes, 16), dtype=torch.uint8, device=self.device)
+            self._host.copy_to_device(dev.data_ptr())
+            self._dev = dev
+        return self._dev
+
+    def in_launch(self, K, stream: int):
+        """What a launch on that stream carries: the plan itself, or None where it reads the device buffer."""
+        return self._host if self._dev is None and not K.kvt_stream_capturing(stream) else None
 
     @property
     def reqs_ptr(self) -> int:
@@ -153,17 +171,22 @@ class AttnTransfer:
             return
         if layer_end is None:
             layer_end = self.num_layers
-        s = stream.cuda_stream if stream is not None else torch.cuda.current_stream(self.device).cuda_stream
+        if stream is not None:
+            s = stream.cuda_stream
+        else:
+            index = self.device.index
+            s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+        carried = plan.in_launch(self.K, s)
         tma = self.use_tma if use_tma is None else (use_tma and self.use_tma)
         hm = self.head_map
         self.K.kvt_launch_p2d_attn(
             self.src_layers.data_ptr(), self.dst_layers.data_ptr(),
             self.src_maps.data_ptr() if tma else 0, self.dst_maps.data_ptr() if tma else 0,
-            self.src_kvt, self.dst_kvt, layer_begin, layer_end, plan.reqs_ptr, plan.n_reqs, plan.total_tiles,
-            plan.block_ids_ptr, self.tile_tokens, hm.src_head0, hm.dst_head0, hm.n_heads, self.mode,
+            self.src_kvt, self.dst_kvt, layer_begin, layer_end, 0 if carried else plan.reqs_ptr, plan.n_reqs, plan.total_tiles,
+            0 if carried else plan.block_ids_ptr, self.tile_tokens, hm.src_head0, hm.dst_head0, hm.n_heads, self.mode,
             self.status.data_ptr(), self.status.data_ptr() + 8 if flag_ptr else 0, flag_ptr, flag_value,
             grid, threads, 1 if tma else 0, s, self.simt_tile, 1 if self.dst_remote else 0, self.tile_order,
-            self.store_form, self.tma_stages, self.cache_hint)
+            self.store_form, self.tma_stages, self.cache_hint, carried)
 
     def check_status(self) -> Tuple[int, int]:
         st = self.status[:2].tolist()
