@@ -30,6 +30,50 @@ namespace py = pybind11;
 
 namespace kvx {
 
+// A request's block tables as an argument: lists of plain ints are read directly, whatever else is converted as before.
+struct BlockTables {
+  BlockIds ids;
+  bool read(PyObject* tables) {
+    if (!PyList_CheckExact(tables)) return false;
+    ids.resize(static_cast<size_t>(PyList_GET_SIZE(tables)));
+    for (size_t g = 0; g < ids.size(); ++g) {
+      PyObject* table = PyList_GET_ITEM(tables, static_cast<Py_ssize_t>(g));
+      if (!PyList_CheckExact(table)) return false;
+      const Py_ssize_t n = PyList_GET_SIZE(table);
+      ids[g].resize(static_cast<size_t>(n));
+      for (Py_ssize_t i = 0; i < n; ++i) {
+        PyObject* id = PyList_GET_ITEM(table, i);
+        if (!PyLong_CheckExact(id)) return false;
+        int beyond = 0;
+        const long long v = PyLong_AsLongLongAndOverflow(id, &beyond);
+        if (beyond != 0 || v < 0 || v > 0xffffffffll) return false;
+        ids[g][static_cast<size_t>(i)] = static_cast<uint32_t>(v);
+      }
+    }
+    return true;
+  }
+};
+
+}  // namespace kvx
+
+namespace pybind11 {
+namespace detail {
+template <>
+struct type_caster<kvx::BlockTables> {
+  PYBIND11_TYPE_CASTER(kvx::BlockTables, make_caster<kvx::BlockIds>::name);
+  bool load(handle src, bool convert) {
+    if (value.read(src.ptr())) return true;
+    make_caster<kvx::BlockIds> any;
+    if (!any.load(src, convert)) return false;
+    value.ids = cast_op<kvx::BlockIds&&>(std::move(any));
+    return true;
+  }
+};
+}  // namespace detail
+}  // namespace pybind11
+
+namespace kvx {
+
 namespace {
 
 struct HybridArgs {
@@ -51,6 +95,7 @@ struct HybridArgs {
   // the worker's cache as a member of an NVLink multicast group: multicast address per [layer][tensor], group size
   std::vector<std::vector<uint64_t>> mc_layers;
   uint32_t mc_size = 0;
+  std::vector<uint64_t> peer_events;     // client: interprocess events, one a layer, beside `events`
 };
 
 void apply_hybrid(WorkerInfo* wi, const HybridArgs& h) {
@@ -134,7 +179,9 @@ class KvClient {
     if (!send_done_addr.empty()) ctx->worker_info_mutable()->ext["sdaddr"] = send_done_addr;
     if (!events.empty()) {
       RTASSERT(events.size() == layers.size());
-      ctx->set_cuda_barrier(std::make_unique<CudaEventBarrier>(events));
+      auto barrier = std::make_unique<CudaEventBarrier>(events, h.peer_events);
+      barrier_ = barrier.get();
+      ctx->set_cuda_barrier(std::move(barrier));
     }
     std::shared_ptr<INamingClient> naming;
     if (!naming_url.empty() && naming_url.rfind("fake", 0) != 0) {
@@ -145,8 +192,21 @@ class KvClient {
     client_ = std::make_unique<KvTransferClient>(std::move(ctx), std::move(factory));
   }
   KvTransferClient* get() { return client_.get(); }
+  // One layer of the forward pass: its event on the engine's stream, and word of it to the open step.
+  void record_layer(size_t stepid, uint64_t event, uint64_t stream) {
+    record_event(event, stream);
+    client_->notify_event_record(stepid, stream);
+  }
+  void share_layer_events() {
+    if (barrier_ != nullptr) barrier_->share();
+  }
+  void record_event(uint64_t event, uint64_t stream) {
+    if (barrier_ != nullptr) barrier_->record(event, stream);
+    else cuda_check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "cudaEventRecord(layer)");
+  }
 
  private:
+  CudaEventBarrier* barrier_{nullptr};    // the context's, which the client owns
   std::unique_ptr<KvTransferClient> client_;
 };
 
@@ -183,16 +243,11 @@ class KvServer {
 std::unique_ptr<KvClient> g_client;
 std::unique_ptr<KvServer> g_server;
 
-KvTransferClient* need_client() {
+KvClient& need_kv_client() {
   if (!g_client) throw KVTransferException(ErrorKind::INVALID_OPERATION, "kv client is not initialized");
-  return g_client->get();
+  return *g_client;
 }
-
-// One layer of the forward pass: its event on the engine's stream, and word of it to the open step.
-void record_layer(KvTransferClient* c, size_t stepid, uint64_t event, uint64_t stream) {
-  cuda_check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "cudaEventRecord(layer)");
-  c->notify_event_record(stepid, stream);
-}
+KvTransferClient* need_client() { return need_kv_client().get(); }
 
 std::optional<WorkerInfo> parse_py_worker_info(const py::handle& h) {
   if (h.is_none()) return std::nullopt;
@@ -229,6 +284,7 @@ HybridArgs hybrid_from_kwargs(const py::kwargs& kw) {
   geti("ple_conv_channel_dims", h.ple_conv_channel_dims);
   geti("mc_layers", h.mc_layers);
   geti("mc_size", h.mc_size);
+  geti("peer_events", h.peer_events);
   return h;
 }
 
@@ -409,12 +465,12 @@ void bind_engine(py::module_& m) {
            py::arg("cache_shape") = -1)
       .def("submit_req_send2",
            [](KvClient& c, const std::string& dst_inst, uint32_t dst_worker, const std::string& reqid, uint32_t seen,
-              uint32_t new_tokens, bool last, const BlockIds& src, const BlockIds& dst, const py::object& info,
+              uint32_t new_tokens, bool last, BlockTables src, BlockTables dst, const py::object& info,
               size_t stepid, uint32_t substepid, uint32_t fanout) {
              std::optional<std::string> s;
              if (!info.is_none()) s = info.cast<std::string>();
-             c.get()->submit_req_send(dst_inst, dst_worker, reqid, seen, new_tokens, last, src, dst, s, stepid, substepid,
-                                      fanout);
+             c.get()->submit_req_send(dst_inst, dst_worker, reqid, seen, new_tokens, last, std::move(src.ids), std::move(dst.ids), s,
+                                      stepid, substepid, fanout);
            },
            py::arg("dst_inst"), py::arg("dst_worker"), py::arg("reqid"), py::arg("seen_tokens"), py::arg("new_tokens"),
            py::arg("has_last_token"), py::arg("src_block_ids"), py::arg("dst_block_ids"),
@@ -438,7 +494,9 @@ void bind_engine(py::module_& m) {
            py::arg("stepid") = 1024, py::arg("sched_tokens") = 1)
       .def("notify_event_record", [](KvClient& c, size_t stepid) { c.get()->notify_event_record(stepid); })
       .def("record_layer",
-           [](KvClient& c, size_t stepid, uint64_t event, uint64_t stream) { record_layer(c.get(), stepid, event, stream); })
+           [](KvClient& c, size_t stepid, uint64_t event, uint64_t stream) { c.record_layer(stepid, event, stream); })
+      .def("share_layer_events", [](KvClient& c) { c.share_layer_events(); }, "As when a peer asks for the layer events.")
+      .def("record_layer_event", [](KvClient& c, uint64_t event, uint64_t stream) { c.record_event(event, stream); })
       .def("flush_send", [](KvClient& c, size_t stepid) { c.get()->flush_send(stepid); })
       .def("drain", [](KvClient& c) { c.get()->drain(); }, py::call_guard<py::gil_scoped_release>())
       .def("wait_inflight",
@@ -526,12 +584,12 @@ void bind_engine(py::module_& m) {
   m.def(
       "submit_req_send2",
       [](const std::string& dst_inst, uint32_t dst_worker, const std::string& reqid, uint32_t seen, uint32_t new_tokens,
-         bool last, const BlockIds& src, const BlockIds& dst, const py::object& info, size_t stepid,
+         bool last, BlockTables src, BlockTables dst, const py::object& info, size_t stepid,
          uint32_t substepid, uint32_t fanout) {
         std::optional<std::string> s;
         if (!info.is_none()) s = info.cast<std::string>();
-        need_client()->submit_req_send(dst_inst, dst_worker, reqid, seen, new_tokens, last, src, dst, s, stepid,
-                                       substepid, fanout);
+        need_client()->submit_req_send(dst_inst, dst_worker, reqid, seen, new_tokens, last, std::move(src.ids), std::move(dst.ids), s,
+                                       stepid, substepid, fanout);
       },
       py::arg("dst_inst"), py::arg("dst_worker"), py::arg("reqid"), py::arg("seen_tokens"), py::arg("new_tokens"),
       py::arg("has_last_token"), py::arg("src_block_ids"), py::arg("dst_block_ids"), py::arg("dst_worker_info") = py::none(),
@@ -548,7 +606,8 @@ void bind_engine(py::module_& m) {
     need_client()->start_send_substep(stepid, substepid, metas);
   });
   m.def("notify_event_record", [](size_t stepid) { need_client()->notify_event_record(stepid); });
-  m.def("record_layer", [](size_t stepid, uint64_t event, uint64_t stream) { record_layer(need_client(), stepid, event, stream); });
+  m.def("record_layer", [](size_t stepid, uint64_t event, uint64_t stream) { need_kv_client().record_layer(stepid, event, stream); });
+  m.def("record_layer_event", [](uint64_t event, uint64_t stream) { need_kv_client().record_event(event, stream); });
   m.def("flush_send", [](size_t stepid) { need_client()->flush_send(stepid); });
   m.def(
       "current_worker_info",

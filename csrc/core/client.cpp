@@ -27,8 +27,38 @@ void KvTransferClient::TargetMgr::submit(std::shared_ptr<Step> step, StepTasks t
         ++n;
       }
   ctx_->inflight().add(n);
-  auto shared_tasks = std::make_shared<StepTasks>(std::move(tasks));
-  mgr_thd_->spawn([this, step = std::move(step), shared_tasks]() mutable { do_submit(step, *shared_tasks); });
+  // Batches for targets that are known go to their senders from here; where a target is to be made first, and behind such a
+  // submission, the manager's thread does it.  Its wake-up is 10 us that the first launch of a step otherwise waits for.
+  bool full;
+  {
+    std::lock_guard<std::mutex> g(mu_);
+    if (queued_ != 0 || !all_known(tasks)) {
+      ++queued_;
+      auto shared_tasks = std::make_shared<StepTasks>(std::move(tasks));
+      mgr_thd_->spawn([this, step = std::move(step), shared_tasks]() mutable {
+        {
+          std::lock_guard<std::mutex> lk(mu_);
+          do_submit(step, *shared_tasks);
+          --queued_;
+        }
+        shrink(static_cast<size_t>(env_txstub_cap()));
+      });
+      return;
+    }
+    do_submit(step, tasks);
+    full = targets_.size() > static_cast<size_t>(env_txstub_cap());
+  }
+  if (full) mgr_thd_->spawn([this] { shrink(static_cast<size_t>(env_txstub_cap())); });
+}
+
+bool KvTransferClient::TargetMgr::all_known(const StepTasks& tasks) const {
+  for (const auto& [inst, per_worker] : tasks.tasks) {
+    auto it = index_.find(inst);
+    if (it == index_.end()) return false;
+    for (const auto& wt : per_worker)
+      if (wt.first >= it->second.size() || !it->second[wt.first].has_value()) return false;
+  }
+  return true;
 }
 
 void KvTransferClient::TargetMgr::drain() {
@@ -90,10 +120,11 @@ void KvTransferClient::TargetMgr::do_submit(std::shared_ptr<Step>& step, StepTas
           target->thread_hint);
     }
   }
-  shrink(static_cast<size_t>(env_txstub_cap()));
 }
 
 void KvTransferClient::TargetMgr::shrink(size_t cap) {
+  std::list<Target> dead;      // taken down behind the lock: closing a channel synchronises streams and unmaps memory
+  std::lock_guard<std::mutex> g(mu_);
   // evict least-recently-used idle targets; stop at the first one still in flight
   while (targets_.size() > cap) {
     Target& victim = targets_.back();
@@ -108,7 +139,7 @@ void KvTransferClient::TargetMgr::shrink(size_t cap) {
       if (!any) index_.erase(it);
     }
     LOG(INFO) << "TargetMgr.shrink: instid=" << inst << " wid=" << wid;
-    targets_.pop_back();
+    dead.splice(dead.end(), targets_, std::prev(targets_.end()));
   }
   n_targets_.store(targets_.size());
 }
@@ -273,6 +304,12 @@ size_t KvTransferClient::start_send(size_t stepid, size_t sched_tokens) {
   if (last_step_guard_) settle_events(*last_step_guard_->step());   // replaced without a flush
   auto step = std::make_shared<Step>(stepid);
   auto guard = std::make_shared<StepGuard>(ctx_.get(), step);
+  if (!pending_buf_.empty()) {        // first, so that the senders wake first
+    StepTasks tmp;
+    std::swap(tmp, pending_buf_);
+    pending_buf_ = StepTasks{};
+    mgr_.submit(step, std::move(tmp));
+  }
   wait_pool_->spawn([guard] {
     fault_inject_sleep(10 * 1000);
     guard->step()->wait_layers_start_ts = SteadyClock::now();
@@ -286,12 +323,6 @@ size_t KvTransferClient::start_send(size_t stepid, size_t sched_tokens) {
     }
     guard->step()->wait_layers_end_ts = SteadyClock::now();
   });
-  if (!pending_buf_.empty()) {
-    StepTasks tmp;
-    std::swap(tmp, pending_buf_);
-    pending_buf_ = StepTasks{};
-    mgr_.submit(step, std::move(tmp));
-  }
   std::vector<StepMetas> parked;
   {
     std::lock_guard<std::mutex> g(coord_lock_);

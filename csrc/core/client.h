@@ -87,8 +87,11 @@ class KvTransferClient {
    private:
     using Iter = std::list<Target>::iterator;
     Target* get_or_create(const RequestInfo& req);
+    bool all_known(const StepTasks& tasks) const;
     void do_submit(std::shared_ptr<Step>& step, StepTasks& tasks);
     void shrink(size_t cap);
+    std::mutex mu_;              // targets_, index_, next_hint_, queued_
+    size_t queued_{0};           // submissions on their way through the manager's thread
     Context* const ctx_;
     std::unique_ptr<ISendStubFactory> factory_;
     std::list<Target> targets_;  // front = most recently used

@@ -6,6 +6,41 @@
 
 namespace kvx {
 
+static void check(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) throw KVTransferException(ErrorKind::CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+CudaEventBarrier::CudaEventBarrier(std::vector<uint64_t> events, std::vector<uint64_t> peer_events)
+    : events_(std::move(events)), peer_events_(std::move(peer_events)) {
+  RTASSERT(peer_events_.empty() || peer_events_.size() == events_.size());
+  for (size_t l = 0; l < peer_events_.size(); ++l) peer_of_[events_[l]] = peer_events_[l];
+}
+
+void CudaEventBarrier::share() {
+  if (peer_events_.empty()) return;
+  std::lock_guard<std::mutex> g(mu_);
+  if (shared_.load(std::memory_order_relaxed)) return;
+  cudaStream_t s = nullptr;
+  check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+  cudaError_t e = cudaSuccess;
+  for (size_t l = 0; l < events_.size() && e == cudaSuccess; ++l) {
+    e = cudaStreamWaitEvent(s, reinterpret_cast<cudaEvent_t>(events_[l]), 0);
+    if (e == cudaSuccess) e = cudaEventRecord(reinterpret_cast<cudaEvent_t>(peer_events_[l]), s);
+  }
+  cudaStreamDestroy(s);
+  check(e, "cudaEventRecord(peer)");
+  shared_.store(true, std::memory_order_release);
+}
+
+void CudaEventBarrier::record(uint64_t event, uint64_t stream) {
+  std::lock_guard<std::mutex> g(mu_);
+  if (shared_.load(std::memory_order_relaxed)) {
+    auto it = peer_of_.find(event);
+    if (it != peer_of_.end()) event = it->second;
+  }
+  check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "cudaEventRecord(layer)");
+}
+
 void CudaEventBarrier::wait(uint32_t layer) {
   RTASSERT(layer < events_.size());
   cudaError_t e = cudaEventSynchronize(reinterpret_cast<cudaEvent_t>(events_[layer]));

@@ -80,6 +80,8 @@ void SendDoneNotifier::round_trip(const std::vector<char>& buf, int resp_size) {
     throw std::runtime_error("rpc send done: invalid response");
 }
 
+bool SendDoneNotifier::enabled() const { return !addr_.empty() || env_send_done_addr() != nullptr; }
+
 void SendDoneNotifier::notify(const std::vector<const ReqSendTask*>& reqs) {
   if (reqs.empty()) return;
   std::lock_guard<std::mutex> g(mu_);
@@ -348,6 +350,17 @@ struct KvSendStub::Impl {
     if (batch.inflight != nullptr) batch.inflight->done(ok);
   }
 
+  // The record of a batch has arrived, or will not any more.
+  void completed(PendingBatch& pb, PollResult r) noexcept {
+    if (r != PollResult::DONE) {
+      LOG(ERROR) << "KVT tx_stub batch failed on completion. DstId=" << stub->dstid() << ",DstWorkerId=" << stub->dstworkerid()
+                 << ",StepIdx=" << pb.batch.step->step_idx << "." << pb.batch.substepid << ',' << pb.flush_out;
+      if (pb.ch) drop_channel.store(true);
+    }
+    finish(pb, r == PollResult::DONE);
+    pb.ch.reset();
+  }
+
   void do_task(std::shared_ptr<PendingBatch> pbp) noexcept {
     PendingBatch& pb = *pbp;
     BatchSendTask& batch = pb.batch;
@@ -409,6 +422,24 @@ struct KvSendStub::Impl {
       finish(pb, ok);
       return;
     }
+    // A batch that is all this stub has on the device, with nothing waiting for this thread: look for its record here for as long as
+    // a short one takes.  The poller's thread would have to be woken first (10 us).  A batch whose end is reported to a scheduler,
+    // or checked, is left to the poller: the answer would hold up the next batch here.
+    if (async && completing.load(std::memory_order_acquire) == 0 && check_ctx == nullptr && (pb.finished_req.empty() || !notifier.enabled())) {
+      const Timepoint until = SteadyClock::now() + std::chrono::microseconds(100);
+      PollResult r = PollResult::PENDING;
+      try {
+        while (r == PollResult::PENDING && !ThreadPool::others_wait() && SteadyClock::now() < until)
+          r = pb.ch->poll_completion(pb.ticket, pb.flush_out);
+      } catch (const std::exception& ex) {
+        LOG(ERROR) << "completion poll failed: " << ex.what();
+        r = PollResult::FAILED;
+      }
+      if (r != PollResult::PENDING) {
+        completed(pb, r);
+        return;
+      }
+    }
     // The batch (or an earlier one of this stub) completes on the device: hand it to the completion poller,
     // which finishes this stub's batches in the order they were sent.
     completing.fetch_add(1, std::memory_order_acq_rel);
@@ -422,14 +453,7 @@ struct KvSendStub::Impl {
       e.poll = [ok] { return ok ? PollResult::DONE : PollResult::FAILED; };
     }
     e.finish = [self, pbp](PollResult r) {
-      if (r != PollResult::DONE) {
-        LOG(ERROR) << "KVT tx_stub batch failed on completion. DstId=" << self->stub->dstid() << ",DstWorkerId="
-                   << self->stub->dstworkerid() << ",StepIdx=" << pbp->batch.step->step_idx << "." << pbp->batch.substepid
-                   << ',' << pbp->flush_out;
-        if (pbp->ch) self->drop_channel.store(true);
-      }
-      self->finish(*pbp, r == PollResult::DONE);
-      pbp->ch.reset();
+      self->completed(*pbp, r);
       self->completing.fetch_sub(1, std::memory_order_acq_rel);
     };
     CompletionPoller::instance().add(std::move(e));

@@ -60,6 +60,7 @@ class SendDoneNotifier {
   // `addr` ("ip:port") overrides BLLM_KVTRANS_SEND_DONE_ADDR; empty = use the environment.
   explicit SendDoneNotifier(uint32_t worker_tp_rank, std::string addr = "") : rank_(worker_tp_rank), addr_(std::move(addr)) {}
   void notify(const std::vector<const ReqSendTask*>& reqs);
+  bool enabled() const;      // notify() talks to somebody
   static std::vector<char> encode(uint32_t worker_tp_rank, const std::vector<const ReqSendTask*>& reqs, int head_kind,
                                   int* resp_size);
 

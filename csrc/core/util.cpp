@@ -111,7 +111,12 @@ ThreadPool::~ThreadPool() {
     if (w->thd.joinable()) w->thd.join();
 }
 
+static thread_local const std::atomic<uint32_t>* t_pending = nullptr;   // of the worker that this thread is
+
+bool ThreadPool::others_wait() { return t_pending != nullptr && t_pending->load(std::memory_order_acquire) > 1; }
+
 void ThreadPool::run(Worker* w, size_t idx) {
+  t_pending = &w->pending;
   std::string nm = name_ + std::to_string(idx);
   pthread_setname_np(pthread_self(), nm.substr(0, 15).c_str());
   for (;;) {

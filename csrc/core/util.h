@@ -69,6 +69,8 @@ class ThreadPool {
   void spawn(std::function<void()> fn, int hint);
   size_t size() const { return workers_.size(); }
   void drain();  // block until every queued task has finished
+  // Asked by a task: is another one waiting for its thread?
+  static bool others_wait();
 
  private:
   struct Worker {

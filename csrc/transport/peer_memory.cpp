@@ -157,7 +157,9 @@ PeerEvents export_peer_events(Context* ctx) {
   ICudaBarrier* b = ctx->cuda_barrier();
   if (b == nullptr || ctx->device_id() < 0) return out;
   cudaSetDevice(ctx->device_id());
+  b->share();
   for (uint32_t l = 0; l < ctx->num_layers(); ++l) {
+
     PeerEvents::One e;
     void* ev = b->event(l);
     if (ev == nullptr) return PeerEvents{out.pid, {}};

@@ -28,6 +28,10 @@ TransferProtocol = _K.TransferProtocol
 
 logger = logging.getLogger("llumnix_kv_b200")
 
+# looked up once: record_event() runs once a layer on the engine's forward thread
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
 DEFAULT_STEPID = 1024
 DEFAULT_SUBSTEPID = 0
 EMPTY_STEP_ID = 9223372036854775807
@@ -215,6 +219,8 @@ class KVTransferClient:
                             gdn_conv_channel_dims, kda_conv_dim_first, hybrid_attn_token_size, kda_page_stride,
                             attn_pack_size, num_ple_layers, ple_block_group, ple_conv_elem_size,
                             ple_conv_state_shape, ple_conv_channel_dims)
+        if self._peer_events:
+            kw["peer_events"] = [ev.cuda_event for ev in self._peer_events]
         if mc_layers is not None and mc_size > 1:
             mc = [[int(a)] if isinstance(a, int) else [int(x) for x in a] for a in mc_layers]
             assert len(mc) == len(layer_addrs) and all(len(a) == len(b) for a, b in zip(mc, layer_addrs))
@@ -234,6 +240,7 @@ class KVTransferClient:
             self._c = _K.KvClient(inst_id, tp_size, worker_id, worker_tp_rank, device_id, block_bytes, token_bytes,
                                   layer_num_blocks, naming_url, self._event_addrs, layer_addrs, ops_protocols,
                                   cache_shape, send_done_addr=send_done_addr, **kw)
+        self._record_layer = _K.record_layer if self._c is None else self._c.record_layer
         self._send_done_addr = None
         if send_done_addr:
             h, p = send_done_addr.rsplit(':', 1)
@@ -247,14 +254,15 @@ class KVTransferClient:
     def _init_events(self):
         if self._device_id >= 0:
             with torch.cuda.device(self._device_id):
-                # interprocess: a decode worker that pulls this cache orders its streams after these events
-                # (CUDA IPC event handles), so nobody's host waits for the forward pass
-                self._events = [torch.cuda.Event(interprocess=True) for _ in range(self._num_layers)]
-                for ev in self._events:
+                # a decode worker that pulls this cache orders its streams after the interprocess ones (CUDA IPC event
+                # handles), so nobody's host waits for the forward pass; until there is one the plain ones serve
+                self._events = [torch.cuda.Event() for _ in range(self._num_layers)]
+                self._peer_events = [torch.cuda.Event(interprocess=True) for _ in range(self._num_layers)]
+                for ev in self._events + self._peer_events:
                     ev.record()
             self._event_addrs = [ev.cuda_event for ev in self._events]
         else:
-            self._events = []
+            self._events, self._peer_events = [], []
             self._event_addrs = []
 
     # ---- engine calls ---------------------------------------------------------------------
@@ -275,12 +283,13 @@ class KVTransferClient:
         if self._events:
             # once per layer on the engine's forward thread: the raw handle of the current stream costs 0.2 us where the Stream
             # object that Event.record() makes costs 3.5, and one native call records and notifies
-            device = torch._C._cuda_getDevice()
+            device = _current_device()
             if stream is None or stream.device_index == device:
-                raw = torch._C._cuda_getCurrentRawStream(device) if stream is None else stream.cuda_stream
-                self._call("record_layer", self._cur_step_id, self._event_addrs[layer_id], raw)
+                raw = _raw_stream(device) if stream is None else stream.cuda_stream
+                self._record_layer(self._cur_step_id, self._event_addrs[layer_id], raw)
                 return
-            self._events[layer_id].record(stream)
+            with torch.cuda.device(stream.device_index):
+                self._call("record_layer_event", self._event_addrs[layer_id], stream.cuda_stream)
         self._call("notify_event_record", self._cur_step_id)
 
     def submit_req_send(self, dst_inst_id, dst_worker_id, req_id, new_tokens, has_last_token, src_block_ids,

@@ -11,6 +11,7 @@ reference's channel ``register_data`` / ``send_data(layer)`` pair
 from __future__ import annotations
 
 import dataclasses
+import functools
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -23,6 +24,7 @@ MODE_MXFP8_TO_BF16 = 2
 REQ_PAD_TAIL = 1
 
 
+@functools.lru_cache(maxsize=None)
 def _ops():
     from llumnix_kv_b200 import kvtransfer_ops
 
