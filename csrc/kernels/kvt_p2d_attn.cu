@@ -885,16 +885,23 @@ __global__ void __launch_bounds__(512, 2) kvt_p2d_attn_kernel(const __grid_const
 // its own loads has 2 KiB of it in flight and comes back to the same DRAM pages many times.  Here warp 0 of a CTA walks the
 // block tables and brings each tile's rows and scale bytes into shared memory with untiled bulk copies, one per run that
 // the source holds contiguously; the other warps convert from shared memory and store straight into the destination.  Tiles
-// pass through a ring of as many stages as fit a sixth of an SM's shared memory, four at most, with a full and an empty mbarrier
-// each: tiles of up to 16 KiB of codes have one or more brought ahead of the one being converted.  Larger ones have a stage
-// alone, and the SM's other CTAs cover the wait for it: 16 heads (32 KiB), 16 layers of 2 x 3000 tokens, 596 MB, 106 us
+// pass through a ring of as many stages as fit the CTA's share of an SM's shared memory, four at most, with a full and an empty
+// mbarrier each: tiles of up to 24 KiB of codes have one or more brought ahead of the one being converted.  Larger ones have a
+// stage alone, and the SM's other CTAs cover the wait for it: 16 heads (32 KiB), 16 layers of 2 x 3000 tokens, 596 MB, 106 us
 // against 174 with a warp per tile and 146 with four; one layer of 300 tokens 12, 60 and 22.  Measured (HND fp8 -> NHD bf16,
 // 8 heads, 32 layers of 3 x ~1334 tokens, 795 MB read and written): 197 us with a warp per tile, 178 with four, 170 with
-// eight, 144 this way (5.5 TB/s); one layer of 300 tokens 34 -> 11 us.  The other direction does not gain (the quantiser's
+// eight, 135 this way (5.9 TB/s); one layer of 300 tokens 34 -> 11 us.  Staging the converted rows too, so that the bulk engine
+// stores them, loses (174 to 206 us at 2 to 4 KiB a warp).  The other direction does not gain (the quantiser's
 // arithmetic fills the same warps: 174 against 158 us at 2 heads, 304 against 283 at 8) and stays with its own loads.
-constexpr uint32_t kConvWarps = 4;                        // converting warps
-constexpr uint32_t kConvThreads = 32u * (1u + kConvWarps);
-constexpr uint32_t kConvCtas = 6;                         // per SM
+//
+// WARPS convert in each of CTAS CTAs per SM: 32 warps a SM either way, which is what keeps HBM busy, in few CTAs with deep stages for
+// large tiles and in many for small ones, whose hand-over the others then hide.  us a launch with 4 warps in 6 CTAs for all / with
+// these: 8 heads, 32 layers of 4003 tokens 138 / 135 (5.9 TB/s), 4 heads 82 / 74, 2 heads of 8000 tokens 86 / 78, 16 heads, 16 layers
+// 140 / 135, 20 heads (40 KiB, too large for a sixth of an SM) 66 / 22.  The other shape: 2 heads 104, 3 heads (6 KiB) 70 against 63.
+// More warps a CTA (10 in 4, 12 in 3, 16 in 2) are slower at every size.
+struct ConvLarge { static constexpr uint32_t WARPS = 8, CTAS = 4; };
+struct ConvSmall { static constexpr uint32_t WARPS = 4, CTAS = 8; };
+constexpr uint32_t kConvLargeTile = 8192;                 // bytes of codes from which a tile is large
 constexpr int kConvStages = 4;
 constexpr uint32_t kConvEnd = 0xffffffffu;                // layer of the slot behind the last tile
 
@@ -937,12 +944,12 @@ struct ConvRows {
   }
 };
 
-template <bool IN_LAUNCH>
-__global__ void __launch_bounds__(kConvThreads, kConvCtas) kvt_p2d_expand_kernel(const __grid_constant__ KvtAttnLaunch p,
-                                                                               const uint32_t n_stages, const uint32_t tile_bytes,
-                                                                               const uint32_t stage_bytes,
-                                                                               const __grid_constant__ PlanParam<IN_LAUNCH> plan_param) {
+template <typename SHAPE, bool IN_LAUNCH>
+__global__ void __launch_bounds__(32u * (1u + SHAPE::WARPS), SHAPE::CTAS)
+    kvt_p2d_expand_kernel(const __grid_constant__ KvtAttnLaunch p, const uint32_t n_stages, const uint32_t tile_bytes,
+                          const uint32_t stage_bytes, const __grid_constant__ PlanParam<IN_LAUNCH> plan_param) {
   extern __shared__ __align__(1024) unsigned char smem[];
+  constexpr uint32_t kConvWarps = SHAPE::WARPS;
   const PlanView<IN_LAUNCH> plan(p, plan_param);
   __shared__ uint64_t full[kConvStages], empty[kConvStages];
   __shared__ ConvSlot slots[kConvStages];
@@ -1137,6 +1144,20 @@ bool quant_staged(const KvtAttnLaunch& a) {
   return stage_env > 0 || (stage_env < 0 && a.dst_remote != 0);
 }
 
+// More than 48 KiB of shared memory, the kernel's own arrays (at most 1 KiB) included, take an opt-in, which is per device and
+// sticky: asked for once per device, and again only for a larger size.
+template <typename KERNEL>
+cudaError_t opt_in(KERNEL kern, size_t smem, std::atomic<size_t> (&granted)[kMaxDevices]) {
+  if (smem <= 47 * 1024) return cudaSuccess;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<size_t>* slot = dev >= 0 && dev < kMaxDevices ? &granted[dev] : nullptr;
+  if (slot != nullptr && slot->load(std::memory_order_relaxed) >= smem) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && slot != nullptr) slot->store(smem, std::memory_order_relaxed);
+  return e;
+}
+
 // The plan as a parameter of the launch.
 template <bool IN_LAUNCH>
 PlanParam<IN_LAUNCH> plan_param(const KvtAttnLaunch& a) {
@@ -1147,48 +1168,50 @@ PlanParam<IN_LAUNCH> plan_param(const KvtAttnLaunch& a) {
 
 // The expansion kernel serves what leaves the way of reading open (simt_tile 0, no threads asked for: its CTAs have one size),
 // in tiles of at least 4 KiB of codes (with 2 KiB, one head, the hand-over of a tile costs more than its reading: 32 layers of
-// 6000 tokens 51 us against 43) of which kConvCtas fit an SM; for the rest it says cudaErrorNotSupported and the SIMT kernel
+// 6000 tokens 51 us against 43) of which its CTAs fit an SM; for the rest it says cudaErrorNotSupported and the SIMT kernel
 // serves it.
-cudaError_t launch_expand(const KvtAttnLaunch& a, int grid_ctas, int threads_asked, int sms, uint64_t total, cudaStream_t stream) {
-  const uint64_t rows = (uint64_t)a.n_heads * a.tile_tokens;
-  const uint64_t tile_bytes = (rows * a.src.head_bytes + 127u) & ~127ull;
-  const uint64_t stage_bytes = tile_bytes + ((rows * (a.src.head_bytes >> 5) + 127u) & ~127ull);
-  const uint64_t budget = kSmemBudget / kConvCtas;
-  if (threads_asked > 0 || simt_choice(a) != 0 || a.dst_remote != 0 || tile_bytes < 4096u || stage_bytes > budget) return cudaErrorNotSupported;
+template <typename SHAPE>
+cudaError_t launch_expand_as(const KvtAttnLaunch& a, int grid_ctas, int sms, uint64_t total, uint64_t tile_bytes, uint64_t stage_bytes,
+                             cudaStream_t stream) {
+  const uint64_t budget = kSmemBudget / SHAPE::CTAS;
+  if (stage_bytes > budget) return cudaErrorNotSupported;
   uint64_t stages = budget / stage_bytes;
   if (stages > (uint64_t)kConvStages) stages = kConvStages;
   uint64_t grid = (uint64_t)grid_ctas;
   if (grid_ctas <= 0) {
     const uint64_t tiles = tile_bytes < (128u << 10) ? (128u << 10) / tile_bytes : 1u;
-    grid = std::max<uint64_t>((uint64_t)kConvCtas * sms, std::min<uint64_t>((total + tiles - 1) / tiles, 1u << 30));
+    grid = std::max<uint64_t>((uint64_t)SHAPE::CTAS * sms, std::min<uint64_t>((total + tiles - 1) / tiles, 1u << 30));
   }
   if (grid > total) grid = total;
-  // at most kSmemBudget / kConvCtas bytes: below the 48 KiB that need no opt-in
+  const size_t smem = stages * stage_bytes;
   const auto go = [&](auto in_launch) {
     constexpr bool kIn = decltype(in_launch)::value;
-    kvt_p2d_expand_kernel<kIn><<<(int)grid, kConvThreads, stages * stage_bytes, stream>>>(a, (uint32_t)stages, (uint32_t)tile_bytes,
-                                                                                         (uint32_t)stage_bytes, plan_param<kIn>(a));
+    static std::atomic<size_t> granted[kMaxDevices];
+    const cudaError_t e = opt_in(kvt_p2d_expand_kernel<SHAPE, kIn>, smem, granted);
+    if (e != cudaSuccess) return e;
+    kvt_p2d_expand_kernel<SHAPE, kIn><<<(int)grid, 32u * (1u + SHAPE::WARPS), smem, stream>>>(
+        a, (uint32_t)stages, (uint32_t)tile_bytes, (uint32_t)stage_bytes, plan_param<kIn>(a));
+    return cudaGetLastError();
   };
-  if (a.plan != nullptr) go(std::true_type{}); else go(std::false_type{});
-  return cudaGetLastError();
+  return a.plan != nullptr ? go(std::true_type{}) : go(std::false_type{});
+}
+
+cudaError_t launch_expand(const KvtAttnLaunch& a, int grid_ctas, int threads_asked, int sms, uint64_t total, cudaStream_t stream) {
+  const uint64_t rows = (uint64_t)a.n_heads * a.tile_tokens;
+  const uint64_t tile_bytes = (rows * a.src.head_bytes + 127u) & ~127ull;
+  const uint64_t stage_bytes = tile_bytes + ((rows * (a.src.head_bytes >> 5) + 127u) & ~127ull);
+  if (threads_asked > 0 || simt_choice(a) != 0 || a.dst_remote != 0 || tile_bytes < 4096u) return cudaErrorNotSupported;
+  return tile_bytes >= kConvLargeTile ? launch_expand_as<ConvLarge>(a, grid_ctas, sms, total, tile_bytes, stage_bytes, stream)
+                                      : launch_expand_as<ConvSmall>(a, grid_ctas, sms, total, tile_bytes, stage_bytes, stream);
 }
 
 template <int MODE, bool USE_TMA, bool IN_LAUNCH>
 cudaError_t launch_as(const KvtAttnLaunch& a, int grid, int threads, uint32_t stages, uint32_t tile_bytes, size_t smem,
                       uint32_t warp_tiles, cudaStream_t stream) {
   auto kern = kvt_p2d_attn_kernel<MODE, USE_TMA, IN_LAUNCH>;
-  if (smem > 48 * 1024) {
-    // the opt-in is per device and sticky: ask once per device (and again only for a larger size)
-    static std::atomic<size_t> granted[kMaxDevices];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::atomic<size_t>* slot = dev >= 0 && dev < kMaxDevices ? &granted[dev] : nullptr;
-    if (slot == nullptr || slot->load(std::memory_order_relaxed) < smem) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      if (slot != nullptr) slot->store(smem, std::memory_order_relaxed);
-    }
-  }
+  static std::atomic<size_t> granted[kMaxDevices];
+  const cudaError_t e = opt_in(kern, smem, granted);
+  if (e != cudaSuccess) return e;
   kern<<<grid, threads, smem, stream>>>(a, stages, tile_bytes, warp_tiles, plan_param<IN_LAUNCH>(a));
   return cudaGetLastError();
 }
