@@ -24,11 +24,20 @@ import ctypes
 import dataclasses
 import hashlib
 import struct
+import threading
 from typing import List, Optional, Sequence, Tuple
 
 import torch
 
 from llumnix_kv_b200.ops.layouts import AttnLayout, CacheShape
+
+# Whole slots that lie beside one another cross PCIe as copies of a copy engine, between the arena and a buffer on the GPU that the
+# transfer kernel fills or empties: an engine moves 57.0 GB/s out and 55.3 in where the SMs store 52.3 and load 51.1, but it wants
+# long runs (4 MiB 52 both ways, 1 MiB 46 and 44).  us a call through the mapping / this way: 24 blocks of 2 MiB saved 998 / 970, 160
+# fp8 blocks of 1 MiB loaded 3471 / 3227 (53.6 GB/s).  Two halves of 16 MiB: a kernel takes 10 us of the 290 that its copy does.
+_STAGE_HALF = 16 << 20       # bytes of each of the two halves, one filled while the other is emptied
+_STAGED_RUN = 8 << 20        # mean run from which the engines are the faster way
+_STAGED_LEAST = 16 << 20     # and the least that a move brings: below, the buffer's own kernel is in the way of too few copies
 
 RESERVE_NEW, RESERVE_EXISTS, RESERVE_BUSY, RESERVE_FULL = 0, 1, 2, 3
 
@@ -105,6 +114,8 @@ class PinnedKVStore:
         self.host = torch.frombuffer(self._buf, dtype=torch.uint8)   # the arena as a CPU tensor
         self._registered = False
         self._save_xfer = self._load_xfer = None
+        self._staging = self._stage_save = self._stage_load = None
+        self.n_slots = n_slots
         self.stream: Optional[torch.cuda.Stream] = None
         if self.device.type == "cuda":
             from llumnix_kv_b200.ops.p2d_attn import MODE_BF16_TO_MXFP8, MODE_COPY, MODE_MXFP8_TO_BF16, AttnTransfer
@@ -124,6 +135,34 @@ class PinnedKVStore:
                 self._load_xfer = AttnTransfer(self.page, engine_layout, page_ptrs, eng_ptrs, self.device,
                                                mode=MODE_MXFP8_TO_BF16 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2)
                 self.uses_tma = tma and self._save_xfer.use_tma and self._load_xfer.use_tma
+                if not tma:
+                    self._init_staging(engine_layout, eng_ptrs, n_slots)
+
+    def _init_staging(self, engine_layout: AttnLayout, eng_ptrs: List[int], n_slots: int) -> None:
+        from llumnix_kv_b200.ops.p2d_attn import MODE_BF16_TO_MXFP8, MODE_COPY, MODE_MXFP8_TO_BF16, AttnTransfer
+
+        if self.slot_bytes > _STAGE_HALF or n_slots * self.slot_bytes < _STAGED_LEAST:
+            return
+        self._stage_slots = min(n_slots, _STAGE_HALF // self.slot_bytes)
+        page = store_page_layout(engine_layout, 2 * self._stage_slots, self.num_layers, self.fp8)
+        try:
+            self._staging = torch.empty(2 * self._stage_slots * self.slot_bytes, dtype=torch.uint8, device=self.device)
+        except torch.cuda.OutOfMemoryError:      # the arena is then reached through its mapping alone
+            return
+        self._copy_stream = torch.cuda.Stream(self.device)
+        for s in (self.stream, self._copy_stream):   # what is under way there outlives a store that is dropped
+            self._staging.record_stream(s)
+        ptrs = [self._staging.data_ptr() + i * self.page_bytes for i in range(self.num_layers)]
+        self._stage_save = AttnTransfer(engine_layout, page, eng_ptrs, ptrs, self.device,
+                                        mode=MODE_BF16_TO_MXFP8 if self.fp8 else MODE_COPY)
+        self._stage_load = AttnTransfer(page, engine_layout, ptrs, eng_ptrs, self.device,
+                                        mode=MODE_MXFP8_TO_BF16 if self.fp8 else MODE_COPY)
+        self._stage_grid = int(os.environ.get("BLLM_KVSTORE_CTAS", "0"))
+        # per half: the kernel is through with it, the copy engine is
+        self._kernel_done = [torch.cuda.Event() for _ in range(2)]
+        self._copy_done = [torch.cuda.Event() for _ in range(2)]
+        self._half = 0
+        self._stage_lock = threading.Lock()
 
     # ---- index ----------------------------------------------------------------------------------
     def keys(self, token_ids: Sequence[int], n_blocks: int) -> List[bytes]:
@@ -179,8 +218,13 @@ class PinnedKVStore:
             with torch.cuda.device(self.device), torch.cuda.stream(self.stream):
                 if after is not None:
                     self.stream.wait_event(after)
-                plan = xfer.plan([chunk], stream=self.stream)
-                xfer.launch(plan, layer_begin, layer_end, stream=self.stream, grid=self.grid)
+                runs = self._runs(list(slots)) if (layer_begin, layer_end) == (0, self.num_layers) else None
+                plan = None
+                if runs is not None:
+                    self._move_staged(save, runs, list(blocks), list(slots))
+                else:
+                    plan = xfer.plan([chunk], stream=self.stream)
+                    xfer.launch(plan, layer_begin, layer_end, stream=self.stream, grid=self.grid)
                 done = torch.cuda.Event()
                 done.record(self.stream)
             done._keepalive = plan      # the plan's device buffers must outlive the kernel
@@ -205,6 +249,50 @@ class PinnedKVStore:
                     es[b] = ps[s]
         return None
 
+    def _runs(self, slots: List[int]) -> Optional[List[Tuple[int, int]]]:
+        """(first index, number) of the runs of neighbouring slots, or None where the mapping is the better way."""
+        if self._staging is None or len(slots) * self.slot_bytes < _STAGED_LEAST:
+            return None
+        most = len(slots) * self.slot_bytes // _STAGED_RUN
+        runs, first = [], 0
+        for i in range(1, len(slots) + 1):
+            if i == len(slots) or slots[i] != slots[i - 1] + 1:
+                if len(runs) == most or not 0 <= slots[first] <= slots[i - 1] < self.n_slots:
+                    return None
+                runs.append((first, i - first))
+                first = i
+        return runs
+
+    def _move_staged(self, save: bool, runs: List[Tuple[int, int]], blocks: Sequence[int], slots: Sequence[int]) -> None:
+        """On self.stream (the kernels) and the copy stream, whose last copies self.stream waits for."""
+        from llumnix_kv_b200.ops.p2d_attn import ReqChunk
+
+        xfer, ntpb, n_half, copy = self._stage_save if save else self._stage_load, self.engine_layout.ntpb, self._stage_slots, self._copy_stream
+        with self._stage_lock:
+            copy.wait_stream(self.stream)
+            for first, n in runs:
+                for at in range(first, first + n, n_half):
+                    k = min(n_half, first + n - at)
+                    half, self._half = self._half, 1 - self._half
+                    staged = list(range(half * n_half, half * n_half + k))
+                    dev, host = self._staging.data_ptr() + half * n_half * self.slot_bytes, self.kv.data_ptr + slots[at] * self.slot_bytes
+                    chunk = ReqChunk(blocks[at:at + k], staged, 0, k * ntpb) if save else ReqChunk(staged, blocks[at:at + k], 0, k * ntpb)
+                    if save:
+                        self.stream.wait_event(self._copy_done[half])
+                        xfer.launch(xfer.plan([chunk], stream=self.stream), stream=self.stream, grid=self._stage_grid)
+                        self._kernel_done[half].record(self.stream)
+                        copy.wait_event(self._kernel_done[half])
+                        self.K.kvt_memcpy_async(host, dev, k * self.slot_bytes, copy.cuda_stream)
+                        self._copy_done[half].record(copy)
+                    else:
+                        copy.wait_event(self._kernel_done[half])
+                        self.K.kvt_memcpy_async(dev, host, k * self.slot_bytes, copy.cuda_stream)
+                        self._copy_done[half].record(copy)
+                        self.stream.wait_event(self._copy_done[half])
+                        xfer.launch(xfer.plan([chunk], stream=self.stream), stream=self.stream, grid=self._stage_grid)
+                        self._kernel_done[half].record(self.stream)
+            self.stream.wait_stream(copy)
+
     def save_layers(self, layer_begin: int, layer_end: int, blocks: Sequence[int], slots: Sequence[int],
                     after=None):
         """Engine cache -> store pages for layers [begin, end).  ``after``: event on the forward
@@ -215,7 +303,7 @@ class PinnedKVStore:
         return self._move(False, layer_begin, layer_end, blocks, slots, after)
 
     def check_status(self) -> None:
-        for x in (self._save_xfer, self._load_xfer):
+        for x in (self._save_xfer, self._load_xfer, self._stage_save, self._stage_load):
             if x is not None:
                 code, detail = x.check_status()
                 if code != 0:
@@ -231,6 +319,7 @@ class PinnedKVStore:
                 self.K.kvt_host_unregister(self.kv.data_ptr)
             self._registered = False
         self._save_xfer = self._load_xfer = None
+        self._staging = self._stage_save = self._stage_load = None
         self.host = None
         self._buf = None
         self.kv = None
