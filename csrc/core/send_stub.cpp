@@ -278,6 +278,7 @@ struct KvSendStub::Impl {
         const size_t rem = num_layers - i, want = std::min(std::max<size_t>(1, ch->preferred_run(rem)), rem);
         batch.step->wait_layer_recorded(i + static_cast<uint32_t>(want) - 1);
       } else {
+        if (!batch.step->layer_ready(i)) ch->settle();
         batch.step->wait_layer_ready(i);
       }
       pb.wait_us += w.get_elapse_us();

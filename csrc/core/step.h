@@ -33,6 +33,7 @@ class Step {
   ~Step();
 
   void wait_layer_ready(uint32_t layer) { want_ready(); data_signal_.wait(layer); }
+  bool layer_ready(uint32_t layer) { return data_signal_.value() > layer; }
   bool wait_layer_ready_for(uint32_t layer, std::chrono::milliseconds d) { want_ready(); return data_signal_.wait_for(layer, d); }
   // A host-driven transport is going to follow ready(i) layer by layer.  Without it the wait-layers thread sleeps until
   // every layer has been recorded and then waits for the last event alone: its waits for the others would contend for

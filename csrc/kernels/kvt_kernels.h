@@ -257,6 +257,11 @@ int kvt_launch_copy_blocks(uint64_t src_base, uint64_t dst_base, const uint64_t*
                            uint32_t n, uint64_t src_capacity, uint64_t dst_capacity,
                            uint32_t* status, int grid_ctas, void* stream);
 
+// The same with the descriptors in HOST memory, read before the call returns: they travel in the launch's parameters.
+#define KVT_CARRIED_DESCS 144u
+int kvt_launch_copy_blocks_carried(uint64_t src_base, uint64_t dst_base, const uint64_t* host_triples, uint32_t n,
+                                   uint64_t src_capacity, uint64_t dst_capacity, uint32_t* status, int grid_ctas, void* stream);
+
 // Gather with the reference's unscaled cast (kvtransfer/src/copy_kernels.cu:369-481): descriptor
 // {src_off, dst_off, n} reads n bf16 values (2n bytes) at src_off and writes n e4m3 bytes at dst_off,
 // round to nearest even, saturating to +-448, NaN kept.  Used by the host-staged transports when

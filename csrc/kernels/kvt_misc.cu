@@ -116,10 +116,27 @@ __global__ void __launch_bounds__(512) kvt_p2d_state_kernel(const __grid_constan
 // SM as well as many short ones do.
 constexpr uint32_t kCopySeg = 4096;
 
+// The descriptors are in memory, or a short list of them in the launch's own parameters (CARRIED): a list that is used once then
+// needs no upload, which on the receiving end of a transfer would queue behind the copy that brings the data.  The lanes of a warp
+// read one descriptor together, by its generic address.  32 layers of 4 MiB through shared memory: 4.42 ms with uploads, 4.23 this way.
+template <bool CARRIED>
+struct DescParam {};
+template <>
+struct DescParam<true> {
+  uint64_t t[3u * KVT_CARRIED_DESCS];
+};
+
+template <bool CARRIED>
 __global__ void __launch_bounds__(512) kvt_copy_blocks_kernel(const char* __restrict__ src, char* __restrict__ dst,
-                                                               const uint64_t* __restrict__ triples, uint32_t n,
-                                                               uint64_t src_cap, uint64_t dst_cap,
-                                                               uint32_t* status) {
+                                                               const uint64_t* in_memory, uint32_t n,
+                                                               uint64_t src_cap, uint64_t dst_cap, uint32_t* status,
+                                                               const __grid_constant__ DescParam<CARRIED> carried) {
+  const uint64_t* triples = in_memory;
+  if constexpr (CARRIED) {
+    uint64_t at = reinterpret_cast<uint64_t>(&carried.t[0]);
+    asm volatile("" : "+l"(at));
+    triples = reinterpret_cast<const uint64_t*>(at);
+  }
   const uint32_t warps_per_cta = blockDim.x >> 5;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const uint64_t len0 = triples[2];
@@ -275,9 +292,21 @@ extern "C" int kvt_launch_copy_blocks(uint64_t src_base, uint64_t dst_base, cons
                                       int grid_ctas, void* stream) {
   if (n == 0) return (int)cudaSuccess;
   // two CTAs of 512 threads per SM by default: a warp keeps 2 KiB in flight
-  kvt_copy_blocks_kernel<<<grid_ctas > 0 ? grid_ctas : 2 * pick_grid(0), 512, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  kvt_copy_blocks_kernel<false><<<grid_ctas > 0 ? grid_ctas : 2 * pick_grid(0), 512, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const char*>(src_base), reinterpret_cast<char*>(dst_base), triples, n, src_capacity,
-      dst_capacity, status);
+      dst_capacity, status, DescParam<false>{});
+  return (int)cudaGetLastError();
+}
+
+extern "C" int kvt_launch_copy_blocks_carried(uint64_t src_base, uint64_t dst_base, const uint64_t* host_triples, uint32_t n,
+                                              uint64_t src_capacity, uint64_t dst_capacity, uint32_t* status, int grid_ctas,
+                                              void* stream) {
+  if (n == 0) return (int)cudaSuccess;
+  if (n > KVT_CARRIED_DESCS) return (int)cudaErrorInvalidValue;
+  DescParam<true> d;
+  memcpy(d.t, host_triples, (size_t)n * 24u);
+  kvt_copy_blocks_kernel<true><<<grid_ctas > 0 ? grid_ctas : 2 * pick_grid(0), 512, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const char*>(src_base), reinterpret_cast<char*>(dst_base), nullptr, n, src_capacity, dst_capacity, status, d);
   return (int)cudaGetLastError();
 }
 

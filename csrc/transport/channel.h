@@ -32,6 +32,8 @@ class IChannel {
   virtual bool device_ordered() const { return false; }
   // May be asynchronous; flush() blocks until every send_data of the batch has landed.
   virtual void send_data(size_t layer_index, Step* step) = 0;
+  // The next layer is not ready yet: whatever the channel holds back until then is better sent now.
+  virtual void settle() {}
   // Every layer of [begin, end) at once, for steps whose data is already complete.  Return
   // false to be driven layer by layer through send_data().
   virtual bool send_layers(size_t layer_begin, size_t layer_end, Step* step) {

@@ -9,6 +9,8 @@
 #include <string>
 #include <vector>
 
+#include "kernels/kvt_kernels.h"
+
 namespace kvx {
 
 struct Triple {
@@ -55,6 +57,24 @@ class DeviceStage {
                uint64_t dst_cap, int grid_ctas = 0, int host_side = HOST_NONE, bool cast_bf16_e4m3 = false);
   uint64_t memcpy_lists() const { return memcpy_lists_; }   // lists that went to the copy engines
   uint64_t kernel_lists() const { return kernel_lists_; }
+  // Pinned host memory -> scattered runs.  A list whose source is one dense run crosses PCIe as copies of the copy engine into this
+  // stage's own buffer, from where the kernel scatters it; any other list, or a short one, is read through the mapping.
+  void enqueue_from_host(uint64_t src_base, uint64_t dst_base, const std::vector<Triple>& triples, uint64_t src_cap, uint64_t dst_cap);
+  // Lists that several launches use: uploaded once by keep() (after forget(), with nothing enqueued still running; it returns the
+  // list's place), then enqueued between whatever bases their offsets are meant for.  `triples` is the same list.
+  void forget(size_t lists_total);
+  size_t keep(const std::vector<Triple>& triples);
+  void enqueue_kept(uint64_t src_base, uint64_t dst_base, size_t place, const std::vector<Triple>& triples, uint64_t src_cap,
+                    uint64_t dst_cap, int host_side, bool cast_bf16_e4m3);
+  void reserve_staging(size_t bytes);
+  static constexpr size_t kStagingLeast = 512u << 10, kStagingMax = 8u << 20;
+  // A mark is a completion record in mapped host memory behind everything enqueued so far; at most kMarks are open, and they are
+  // waited for in order.  wait_mark() returns when it has arrived and throws as sync() does; poll_mark() says whether it has.
+  static constexpr size_t kMarks = 8;
+  uint64_t mark();
+  bool poll_mark(uint64_t m);
+  void wait_mark(uint64_t m);
+  void quiesce() noexcept;      // nothing enqueued is running any more, however it ended
   // Wait for everything enqueued and throw KVTransferException if the kernel flagged a descriptor.
   void sync();
   void* stream() const { return stream_; }
@@ -66,15 +86,35 @@ class DeviceStage {
   void* record_done();
 
  private:
+  // Descriptors [place, place + n) of d_triples_.
+  void launch_list(uint64_t src_base, uint64_t dst_base, size_t place, size_t n, uint64_t src_cap, uint64_t dst_cap, int grid_ctas,
+                   int host_side, bool cast);
+  bool copy_engines(uint64_t src_base, uint64_t dst_base, const std::vector<Triple>& triples, uint64_t src_cap, uint64_t dst_cap,
+                    int host_side);
+  void launch_new(uint64_t src_base, uint64_t dst_base, const Triple* triples, size_t n, uint64_t src_cap, uint64_t dst_cap,
+                  int grid_ctas, int host_side, bool cast);
+  int copy_grid(int grid_ctas, int host_side) const;
+  static uint64_t dense_source(const std::vector<Triple>& triples, uint64_t src_cap);
+  size_t upload(const Triple* triples, size_t n);
+  void make_room(size_t n);
+
   int device_;
   void* stream_{nullptr};
   void* done_event_{nullptr};
   uint64_t* d_triples_{nullptr};
   size_t d_cap_{0};       // triples
   size_t used_{0};        // triples enqueued since the last sync
+  size_t kept_{0};        // the first of them, which stay
   uint32_t* d_status_{nullptr};
   PinnedBuffer h_triples_;
   PinnedBuffer h_status_;
+  static constexpr size_t kMarksAt = 64;
+  KvtCompletion* h_marks_{nullptr};      // kMarks records, behind the status words
+  KvtCompletion* d_marks_{nullptr};
+  uint64_t marks_{0}, waited_{0};        // enqueued, waited for
+  uint32_t polls_{0};
+  char* d_staging_{nullptr};
+  size_t staging_cap_{0};
   uint64_t memcpy_lists_{0};
   uint64_t kernel_lists_{0};
 };

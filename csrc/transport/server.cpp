@@ -23,6 +23,7 @@
 #include <unistd.h>
 
 #include <atomic>
+#include <deque>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -151,6 +152,41 @@ class TransferServer : public ITransferServer {
     return std::min<size_t>(lim, 0xffffffffu);
   }
 
+  // A layer whose scatter is enqueued and not answered yet.
+  struct Owed {
+    uint64_t mark;
+    uint64_t reqid;
+    Timepoint t_start;
+  };
+  static constexpr size_t kOwedMost = 2;      // of DeviceStage::kMarks
+
+  // Something has arrived on the connection, its end included.
+  static bool data_frame_waits(int cfd) {
+    struct pollfd p{cfd, POLLIN, 0};
+    return ::poll(&p, 1, 0) > 0;
+  }
+
+  // Answers the oldest layer owed if its scatter has ended (`wait`: when it has).  False: the connection is gone.
+  bool settle_one(int cfd, std::mutex& write_mu, DeviceStage& stage, std::deque<Owed>& owed, bool wait) {
+    const Owed o = owed.front();
+    uint32_t status = WIRE_OK;
+    try {
+      if (wait) {
+        stage.wait_mark(o.mark);
+      } else if (!stage.poll_mark(o.mark)) {
+        std::this_thread::yield();
+        return true;
+      }
+    } catch (const std::exception& ex) {
+      LOG(ERROR) << "KVT server scatter failed,reqid=" << o.reqid << ",ex=" << ex.what();
+      status = WIRE_INTERNAL;
+    }
+    owed.pop_front();
+    const std::string resp = data_reply(o.reqid, status, o.t_start);
+    std::lock_guard<std::mutex> wg(write_mu);
+    return send_frame(cfd, resp.data(), resp.size(), env_rpc_timeout_s() * 1000);
+  }
+
   void serve(int cfd) {
     FdGuard fd(cfd);
     std::unique_ptr<DeviceStage> stage;
@@ -160,11 +196,17 @@ class TransferServer : public ITransferServer {
     // a pull session answers finished batches from the completion thread: every write to this connection is locked
     auto write_mu = std::make_shared<std::mutex>();
     std::shared_ptr<PullSession> pull;
+    std::deque<Owed> owed;
     const size_t frame_max = frame_limit();
     try {
       if (gpu) stage = std::make_unique<DeviceStage>(ctx_->device_id());
       for (;;) {
         uint32_t n = 0;
+        // A scatter out of shared memory that is still under way is answered as it ends, but the next layer's frame, when it is
+        // here before that, is taken first: its scatter then follows without a gap.
+        bool gone = false;
+        while (!owed.empty() && !gone && (owed.size() >= kOwedMost || !data_frame_waits(cfd))) gone = !settle_one(cfd, *write_mu, *stage, owed, false);
+        if (gone) break;
         // Idle connections block here; stop() shuts the socket down to wake them.
         if (read_full(cfd, &n, 4, 0) != 4) break;
         if (n > frame_max) {      // nothing is pinned or read for a length no sender of ours produces
@@ -177,20 +219,26 @@ class TransferServer : public ITransferServer {
         uint32_t magic = 0;
         memcpy(&magic, buf, 4);
         std::string resp;
+        while (magic != KV_CACHE_SHM_MAGIC && !owed.empty() && !gone) gone = !settle_one(cfd, *write_mu, *stage, owed, true);
+        if (gone) break;
         if (magic == KV_CACHE_DATA_MAGIC) {
           uint64_t reqid = 0;
           if (n < RPC_HEADER) break;
           get_rpc_header(buf, &magic, &reqid);
-          resp = on_data(reqid, buf + RPC_HEADER, n - RPC_HEADER, buf, rx.device_ptr(), n, stage.get(), false, 0);
+          resp = on_data(reqid, buf + RPC_HEADER, n - RPC_HEADER, buf, rx.device_ptr(), n, stage.get(), false, 0, nullptr);
         } else if (magic == KV_CACHE_SHM_MAGIC) {
           uint64_t reqid = 0, seg_off = 0;
           if (n < RPC_HEADER + 8) break;
           get_rpc_header(buf, &magic, &reqid);
           memcpy(&seg_off, buf + RPC_HEADER, 8);
           resp = on_data(reqid, buf + RPC_HEADER + 8, n - RPC_HEADER - 8, shm.base, shm.dev, shm.bytes, stage.get(),
-                         true, seg_off);
+                         true, seg_off, &owed);
+          if (resp.empty()) continue;     // answered when it has landed
+          while (!owed.empty() && !gone) gone = !settle_one(cfd, *write_mu, *stage, owed, true);
+          if (gone) break;
         } else if (magic == SHM_ATTACH_REQ) {
           resp = on_attach(buf, n, shm, gpu);
+          if (stage != nullptr && shm.registered) stage->reserve_staging(shm.bytes / 4);   // or the first frame waits for it
         } else if (magic == MEM_HANDLES_REQ) {
           resp = on_mem_handles(buf, n);
         } else if (magic == PULL_OPEN_REQ) {
@@ -236,25 +284,29 @@ class TransferServer : public ITransferServer {
       // the descriptor is about to close: wait (bounded) until nothing can write to it any more
       std::lock_guard<std::mutex> wg(*write_mu);
     }
+    if (stage != nullptr) stage->quiesce();     // a scatter that nobody waited for may still read the segment
     shm.reset();
     std::lock_guard<std::mutex> g(mu_);
     conns_.erase(cfd);
   }
 
+  static std::string data_reply(uint64_t reqid, uint32_t status, Timepoint t_start) {
+    std::string resp(RPC_HEADER, '\0');
+    put_rpc_header(resp.data(), KV_CACHE_DATA_MAGIC, reqid);
+    put(resp, status);
+    put(resp, static_cast<int64_t>(elapse_us(t_start, SteadyClock::now())));
+    return resp;
+  }
+
   // body: the 'KVCa' message after its RPC header ([layer][num_tensors] + per-tensor metadata
   // [+ blob when !external]).  blob_host/blob_dev/blob_cap: the memory the blobs are read from
   // (the received frame itself, or the attached shm segment).
+  // `owed`: the scatter is only enqueued, the answer is noted there for when it has ended, and "" is returned.
   std::string on_data(uint64_t reqid, const char* body, size_t len, const char* blob_host, uint64_t blob_dev,
-                      size_t blob_cap, DeviceStage* stage, bool external, uint64_t seg_off) {
+                      size_t blob_cap, DeviceStage* stage, bool external, uint64_t seg_off, std::deque<Owed>* owed) {
     const auto t_start = SteadyClock::now();
     std::string resp;
-    auto reply = [&](uint32_t status) {
-      resp.resize(RPC_HEADER);
-      put_rpc_header(resp.data(), KV_CACHE_DATA_MAGIC, reqid);
-      put(resp, status);
-      put(resp, static_cast<int64_t>(elapse_us(t_start, SteadyClock::now())));
-      return resp;
-    };
+    auto reply = [&](uint32_t status) { return data_reply(reqid, status, t_start); };
     const char* p = body;
     const char* end = body + len;
     if (len < 2 * sizeof(size_t)) return reply(WIRE_BAD_REQUEST);
@@ -304,13 +356,20 @@ class TransferServer : public ITransferServer {
           cursor += blen;
         }
         if (stage != nullptr) {
-          stage->enqueue(blob_dev, addrs[layer][t], triples, blob_cap, cap, 0, DeviceStage::HOST_SRC);
+          stage->enqueue_from_host(blob_dev, addrs[layer][t], triples, blob_cap, cap);
         } else {
           char* dst = reinterpret_cast<char*>(addrs[layer][t]);
           for (const auto& tr : triples) memcpy(dst + tr.dst_off, blob_host + tr.src_off, tr.len);
         }
       }
-      if (stage != nullptr) stage->sync();
+      if (stage != nullptr) {
+        const uint64_t m = stage->mark();
+        if (owed != nullptr) {
+          owed->push_back(Owed{m, reqid, t_start});
+          return resp;
+        }
+        stage->wait_mark(m);
+      }
     } catch (const std::exception& ex) {
       LOG(ERROR) << "KVT server scatter failed,reqid=" << reqid << ",ex=" << ex.what();
       return reply(WIRE_INTERNAL);
