@@ -216,7 +216,7 @@ void DeviceStage::launch_new(uint64_t src_base, uint64_t dst_base, const Triple*
   launch_list(src_base, dst_base, place, n, src_cap, dst_cap, grid_ctas, host_side, cast);
 }
 
-// The bytes of a list whose source is one dense run of at least kStagingLeast; 0 for any other.
+// The bytes of a list whose source is one dense run that is worth staging; 0 for any other.
 uint64_t DeviceStage::dense_source(const std::vector<Triple>& triples, uint64_t src_cap) {
   uint64_t total = 0;
   for (const Triple& t : triples) {
@@ -224,7 +224,7 @@ uint64_t DeviceStage::dense_source(const std::vector<Triple>& triples, uint64_t 
     total += t.len;
   }
   const uint64_t first = triples[0].src_off;
-  return total < kStagingLeast || first > src_cap || total > src_cap - first ? 0 : total;
+  return total < kStagingLeast || total > kStagingMax || first > src_cap || total > src_cap - first ? 0 : total;
 }
 
 void DeviceStage::reserve_staging(size_t bytes) {
@@ -232,7 +232,7 @@ void DeviceStage::reserve_staging(size_t bytes) {
   if (bytes <= staging_cap_) return;
   cuda_check(cudaSetDevice(device_), "cudaSetDevice");
   void* p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {      // no room: a smaller buffer serves too, and without one the lists go through the mapping
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {      // no room: the lists go through the mapping
     cudaGetLastError();
     return;
   }
@@ -247,7 +247,8 @@ void DeviceStage::reserve_staging(size_t bytes) {
 // A copy engine brings host memory at 55.3 GB/s where the loads of the SMs reach 51.1, and beside SM stores in the other direction, as
 // on a GPU that is sender and receiver, 38 GB/s each way against 35 (4 MiB a copy).  It wants long runs (1 MiB 44.5 GB/s, 64 KiB 12):
 // a frame's blob is one and a layer's pages are not, hence one copy of the blob into a buffer on this GPU and a kernel from there to
-// the pages (4 MiB: 5 us).
+// the pages (4 MiB: 5 us).  The buffer holds the whole blob or is not used: in pieces of 8 MiB, each copied when the one before had been
+// scattered, 32 MiB a layer took 37.0 ms a step, through the mapping 30.1, whole 27.1 (16 MiB: 17.8, 14.9, 14.9).
 void DeviceStage::enqueue_from_host(uint64_t src_base, uint64_t dst_base, const std::vector<Triple>& triples, uint64_t src_cap,
                                     uint64_t dst_cap) {
   if (triples.empty()) return;
@@ -257,33 +258,17 @@ void DeviceStage::enqueue_from_host(uint64_t src_base, uint64_t dst_base, const 
   g_kernel_lists++;
   const uint64_t total = dense_source(triples, src_cap);
   if (total != 0) reserve_staging(total);
-  if (total == 0 || staging_cap_ < kStagingLeast) {
+  if (total == 0 || staging_cap_ < total) {
     launch_new(src_base, dst_base, triples.data(), triples.size(), src_cap, dst_cap, 0, HOST_SRC, false);
     return;
   }
-  // in pieces of what the buffer holds; a descriptor that crosses the end of one is cut there
-  std::vector<Triple> piece;
-  piece.reserve(triples.size());
-  uint64_t from = triples[0].src_off, bytes = 0;
-  const auto move_piece = [&] {
-    cuda_check(cudaMemcpyAsync(d_staging_, reinterpret_cast<const void*>(src_base + from), bytes, cudaMemcpyDefault,
-                               static_cast<cudaStream_t>(stream_)),
-               "cudaMemcpyAsync(staging)");
-    launch_new(reinterpret_cast<uint64_t>(d_staging_), dst_base, piece.data(), piece.size(), staging_cap_, dst_cap, 0, HOST_NONE, false);
-    from += bytes;
-    bytes = 0;
-    piece.clear();
-  };
-  for (const Triple& t : triples) {
-    for (uint64_t done = 0; done < t.len;) {
-      const uint64_t len = std::min<uint64_t>(t.len - done, staging_cap_ - bytes);
-      piece.push_back(Triple{bytes, t.dst_off + done, len});
-      bytes += len;
-      done += len;
-      if (bytes == staging_cap_) move_piece();
-    }
-  }
-  if (bytes != 0) move_piece();
+  const uint64_t from = triples[0].src_off;
+  cuda_check(cudaMemcpyAsync(d_staging_, reinterpret_cast<const void*>(src_base + from), total, cudaMemcpyDefault,
+                             static_cast<cudaStream_t>(stream_)),
+             "cudaMemcpyAsync(staging)");
+  std::vector<Triple> local(triples);
+  for (Triple& t : local) t.src_off -= from;
+  launch_new(reinterpret_cast<uint64_t>(d_staging_), dst_base, local.data(), local.size(), total, dst_cap, 0, HOST_NONE, false);
 }
 
 void DeviceStage::forget(size_t lists_total) {

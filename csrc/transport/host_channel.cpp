@@ -79,6 +79,9 @@ class HostChannel : public IChannel {
     }
     if (use_shm_) ensure_shm(sb_total_ * std::max<size_t>(1, ctx_->num_layers() > 4 ? 4 : ctx_->num_layers()));
     if (ahead()) {
+      // The ring starts over: every frame before has been answered.  Slots of one length that begin at 0 never overlap, which is what
+      // lets a layer be gathered when as many as all slots but one are unanswered; behind a batch of other lengths they would.
+      shm_cursor_ = 0;
       // one list a tensor for all layers of the batch, its destinations counted from the tensor's blob
       kept_.clear();
       stage_->forget(merged_blocks_);
