@@ -43,7 +43,7 @@ void CudaEventBarrier::record(uint64_t event, uint64_t stream) {
 
 void CudaEventBarrier::wait(uint32_t layer) {
   RTASSERT(layer < events_.size());
-  cudaError_t e = cudaEventSynchronize(reinterpret_cast<cudaEvent_t>(events_[layer]));
+  cudaError_t e = cudaEventSynchronize(static_cast<cudaEvent_t>(event(layer)));      // once shared, the plain ones are of earlier steps
   if (e != cudaSuccess) {
     throw KVTransferException(ErrorKind::CUDA, std::string("cudaEventSynchronize: ") + cudaGetErrorString(e));
   }
