@@ -159,7 +159,6 @@ PeerEvents export_peer_events(Context* ctx) {
   cudaSetDevice(ctx->device_id());
   b->share();
   for (uint32_t l = 0; l < ctx->num_layers(); ++l) {
-
     PeerEvents::One e;
     void* ev = b->event(l);
     if (ev == nullptr) return PeerEvents{out.pid, {}};
