@@ -258,8 +258,9 @@ class KVTransferClient:
                 # handles), so nobody's host waits for the forward pass; until there is one the plain ones serve
                 self._events = [torch.cuda.Event() for _ in range(self._num_layers)]
                 self._peer_events = [torch.cuda.Event(interprocess=True) for _ in range(self._num_layers)]
+                stream = torch.cuda.current_stream()      # looked up once, not for each event
                 for ev in self._events + self._peer_events:
-                    ev.record()
+                    ev.record(stream)
             self._event_addrs = [ev.cuda_event for ev in self._events]
         else:
             self._events, self._peer_events = [], []
