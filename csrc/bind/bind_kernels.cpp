@@ -178,9 +178,10 @@ void bind_kernels(py::module_& m) {
       .def_readonly("pool_offset", &HostPlan::pool_offset)
       .def_property_readonly("nbytes", [](const HostPlan& p) { return p.blob.size(); })
       .def_property_readonly("blob", [](const HostPlan& p) { return py::bytes(p.blob); })
-      .def("copy_to_device", [](const HostPlan& p, uint64_t dst) {
-        if (!p.blob.empty()) check_cuda(kvt_copy_now(dst, p.blob.data(), p.blob.size()), "kvt_copy_now");
-      }, "The plan at a device address, complete on return and outside of any capture.");
+      .def("copy_to_device", [](const HostPlan& p, uint64_t dst, uint64_t after) {
+        if (!p.blob.empty()) check_cuda(kvt_copy_now(dst, p.blob.data(), p.blob.size(), reinterpret_cast<void*>(after)), "kvt_copy_now");
+      }, py::arg("dst"), py::arg("after"), py::call_guard<py::gil_scoped_release>(),
+           "The plan at a device address, behind the event `after`, complete on return and outside of any capture.");
   m.def("kvt_pack_chunks", &pack_chunks, py::arg("chunks"), py::arg("tile_tokens"), py::arg("dst_ntpb"));
   m.def("kvt_stream_capturing", [](uint64_t stream) { return kvt_stream_capturing(reinterpret_cast<void*>(stream)) != 0; });
 

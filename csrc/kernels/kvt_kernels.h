@@ -438,8 +438,9 @@ int kvt_host_register(uint64_t host_ptr, uint64_t bytes, uint64_t* dev_ptr);
 int kvt_host_unregister(uint64_t host_ptr);
 // 1: the stream is being captured into a graph.
 int kvt_stream_capturing(void* stream);
-// host -> device copy that is complete on return and stays out of any capture that is going on.
-int kvt_copy_now(uint64_t dst, const void* src, uint64_t bytes);
+// host -> device copy that is complete on return and stays out of any capture that is going on.  `after` (a cudaEvent_t or NULL): what
+// it must not overtake, recorded outside of any capture.
+int kvt_copy_now(uint64_t dst, const void* src, uint64_t bytes, void* after);
 int kvt_sm_count(int dev);
 // Copy-engine copies by raw address (device, peer-mapped or pinned host memory on either side): one
 // cudaMemcpyAsync, or one per {src_off, dst_off, len} triple of a host array.  They are the library

@@ -530,7 +530,7 @@ extern "C" int kvt_stream_capturing(void* stream) {
   return st == cudaStreamCaptureStatusNone ? 0 : 1;
 }
 
-extern "C" int kvt_copy_now(uint64_t dst, const void* src, uint64_t bytes) {
+extern "C" int kvt_copy_now(uint64_t dst, const void* src, uint64_t bytes, void* after) {
   // relaxed for this thread: calls on a stream that nobody captures are then allowed while another stream is being captured
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
@@ -538,7 +538,8 @@ extern "C" int kvt_copy_now(uint64_t dst, const void* src, uint64_t bytes) {
   cudaStream_t s = nullptr;
   e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   if (e == cudaSuccess) {
-    e = cudaMemcpyAsync(reinterpret_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice, s);
+    if (after != nullptr) e = cudaStreamWaitEvent(s, reinterpret_cast<cudaEvent_t>(after), 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(reinterpret_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice, s);
     const cudaError_t w = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = w;
     cudaStreamDestroy(s);
