@@ -218,7 +218,9 @@ class PinnedKVStore:
             with torch.cuda.device(self.device), torch.cuda.stream(self.stream):
                 if after is not None:
                     self.stream.wait_event(after)
-                runs = self._runs(list(slots)) if (layer_begin, layer_end) == (0, self.num_layers) else None
+                runs = None
+                if (layer_begin, layer_end) == (0, self.num_layers) and self._in_cache(blocks):
+                    runs = self._runs(list(slots))
                 plan = None
                 if runs is not None:
                     self._move_staged(save, runs, list(blocks), list(slots))
@@ -248,6 +250,11 @@ class PinnedKVStore:
                 else:
                     es[b] = ps[s]
         return None
+
+    def _in_cache(self, blocks: Sequence[int]) -> bool:
+        """The kernel takes every one of these blocks.  A page that it refuses stays as it was through the mapping; through the
+        buffer the copy behind it would bring the slot whatever an earlier move left there."""
+        return min(blocks) >= 0 and max(blocks) < self.engine_layout.num_blocks
 
     def _runs(self, slots: List[int]) -> Optional[List[Tuple[int, int]]]:
         """(first index, number) of the runs of neighbouring slots, or None where the mapping is the better way."""

@@ -1,0 +1,41 @@
+"""Block ids outside of the cache: their slots stay as they were and the status says so, whichever way a move would have taken."""
+import pytest
+import torch
+
+from llumnix_kv_b200.kvstore import PinnedKVStore
+from llumnix_kv_b200.ops.layouts import AttnLayout, CacheShape
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+LAYERS, N = 8, 70      # slots of 512 KiB: two halves of the buffer and a remainder
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("at", [0, 40, N - 1])
+@pytest.mark.parametrize("bad", [N, 2 ** 32 - 1])
+def test_a_refused_block_leaves_its_slot_alone(ops, fp8, at, bad):
+    lay = AttnLayout(CacheShape.FLASH, N, 16, 8, 128, 2)
+    src = [lay.alloc(DEV, "normal", seed=i) for i in range(LAYERS)]
+    name = "kvx_refused_%d_%d_%d" % (fp8, at, bad)
+    st = PinnedKVStore(name, lay, src, 0, 1, N + 4, create=True, fp8=fp8)
+    try:
+        slots = list(range(2, 2 + N))
+        st.save_layers(0, LAYERS, list(range(N)), slots).synchronize()
+        want = st.host.view(N + 4, st.slot_bytes).clone()
+        assert bool(want[2 + at].any())
+        st.host.fill_(0x5A)
+        blocks = list(range(N))
+        blocks[at] = bad
+        st.save_layers(0, LAYERS, blocks, slots).synchronize()
+        got = st.host.view(N + 4, st.slot_bytes)
+        want[2 + at] = 0x5A
+        assert torch.equal(got[2:2 + N], want[2:2 + N]) and bool((got[:2] == 0x5A).all()) and bool((got[2 + N:] == 0x5A).all())
+        with pytest.raises(RuntimeError, match="status"):
+            st.check_status()
+        kept = [t.clone() for t in src]
+        st.load_layers(0, LAYERS, blocks, slots).synchronize()
+        for t, was in zip(src, kept):      # the block whose id was replaced stays as it was too
+            assert torch.equal(lay.view(t, torch.int16)[at], lay.view(was, torch.int16)[at])
+    finally:
+        st.close()
+        ops.KvStore.unlink(name)
