@@ -80,18 +80,17 @@ static py::tuple pack_plan(const std::vector<std::tuple<std::vector<uint32_t>, s
   return py::make_tuple(py::bytes(p.blob), p.n_reqs, p.total_tiles, p.pool_offset);
 }
 
-// An unsigned 32-bit number: a plain int is read directly, anything else through `convert` (PyNumber_Index or PyNumber_Long).
-static uint32_t as_u32(PyObject* o, PyObject* (*convert)(PyObject*)) {
-  if (!PyLong_CheckExact(o)) {
-    const py::object whole = py::reinterpret_steal<py::object>(convert(o));
-    if (!whole) throw py::error_already_set();
-    if (PyLong_CheckExact(whole.ptr())) return as_u32(whole.ptr(), convert);
-    throw py::type_error("kvt_pack_chunks: not a whole number");
+// An unsigned 32-bit number: a plain int is read directly, anything else converted as an argument of that type is.
+static uint32_t as_u32(PyObject* o) {
+  if (PyLong_CheckExact(o)) {
+    int beyond = 0;
+    const long long v = PyLong_AsLongLongAndOverflow(o, &beyond);
+    if (beyond != 0 || v < 0 || v > 0xffffffffll) throw py::type_error("kvt_pack_chunks: number beyond 32 bits");
+    return static_cast<uint32_t>(v);
   }
-  const unsigned long v = PyLong_AsUnsignedLong(o);
-  if (v == static_cast<unsigned long>(-1) && PyErr_Occurred()) throw py::error_already_set();
-  if (v > 0xffffffffull) throw py::value_error("kvt_pack_chunks: number beyond 32 bits");
-  return static_cast<uint32_t>(v);
+  py::detail::make_caster<uint32_t> any;
+  if (!any.load(o, true)) throw py::type_error("kvt_pack_chunks: not a whole number");
+  return py::detail::cast_op<uint32_t>(any);
 }
 
 // The same from chunk objects (src_blocks, dst_blocks, seen_tokens, new_tokens, pad_tail) without a Python list per table.
@@ -116,15 +115,20 @@ static HostPlan pack_chunks(const py::iterable& chunks, uint32_t tile_tokens, ui
         if (!seq) throw py::error_already_set();
         for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq.ptr()); ++i) {
           const py::object id = py::reinterpret_borrow<py::object>(PySequence_Fast_GET_ITEM(seq.ptr(), i));
-          pool.push_back(as_u32(id.ptr(), &PyNumber_Index));
+          pool.push_back(as_u32(id.ptr()));
         }
       };
     };
-    const py::object seen = attr(kSeen), fresh = attr(kNew), pad = attr(kPad);
+    auto number = [&attr](PyObject* name) {      // int(...) of it
+      const py::object whole = py::reinterpret_steal<py::object>(PyNumber_Long(attr(name).ptr()));
+      if (!whole) throw py::error_already_set();
+      return as_u32(whole.ptr());
+    };
+    const py::object pad = attr(kPad);
     const int padded = PyObject_IsTrue(pad.ptr());
     if (padded < 0) throw py::error_already_set();
-    pk.add(ids(kSrc), ids(kDst), as_u32(seen.ptr(), &PyNumber_Long), as_u32(fresh.ptr(), &PyNumber_Long),
-           padded != 0 ? KVT_REQ_PAD_TAIL : 0u);
+    const uint32_t seen = number(kSeen), fresh = number(kNew);
+    pk.add(ids(kSrc), ids(kDst), seen, fresh, padded != 0 ? KVT_REQ_PAD_TAIL : 0u);
   }
   return pk.finish();
 }
