@@ -68,14 +68,19 @@ struct PlanPacker {
   }
 };
 
-static py::tuple pack_plan(const std::vector<std::tuple<std::vector<uint32_t>, std::vector<uint32_t>, uint32_t,
-                                                        uint32_t, uint32_t>>& reqs,
-                           uint32_t tile_tokens, uint32_t dst_ntpb) {
-  PlanPacker pk{tile_tokens, dst_ntpb, {}, {}};
+// (src_blocks, dst_blocks, seen_tokens, new_tokens, flags)
+using ReqTuple = std::tuple<std::vector<uint32_t>, std::vector<uint32_t>, uint32_t, uint32_t, uint32_t>;
+
+static void add_tuple(PlanPacker& pk, const ReqTuple& r) {
   auto ids = [](const std::vector<uint32_t>& v) {
     return [&v](std::vector<uint32_t>& pool) { pool.insert(pool.end(), v.begin(), v.end()); };
   };
-  for (const auto& r : reqs) pk.add(ids(std::get<0>(r)), ids(std::get<1>(r)), std::get<2>(r), std::get<3>(r), std::get<4>(r));
+  pk.add(ids(std::get<0>(r)), ids(std::get<1>(r)), std::get<2>(r), std::get<3>(r), std::get<4>(r));
+}
+
+static py::tuple pack_plan(const std::vector<ReqTuple>& reqs, uint32_t tile_tokens, uint32_t dst_ntpb) {
+  PlanPacker pk{tile_tokens, dst_ntpb, {}, {}};
+  for (const ReqTuple& r : reqs) add_tuple(pk, r);
   const HostPlan p = pk.finish();
   return py::make_tuple(py::bytes(p.blob), p.n_reqs, p.total_tiles, p.pool_offset);
 }
@@ -94,7 +99,8 @@ static uint32_t as_u32(PyObject* o) {
 }
 
 // The same from chunk objects (src_blocks, dst_blocks, seen_tokens, new_tokens, pad_tail) without a Python list per table.
-static HostPlan pack_chunks(const py::iterable& chunks, uint32_t tile_tokens, uint32_t dst_ntpb) {
+// Objects of another class than `plain` are asked for their tuples: the class may say something else there.
+static HostPlan pack_chunks(const py::iterable& chunks, uint32_t tile_tokens, uint32_t dst_ntpb, const py::handle plain) {
   // the attributes' names, interned once: making them for each chunk took a third of the time
   static PyObject* const kSrc = PyUnicode_InternFromString("src_blocks");
   static PyObject* const kDst = PyUnicode_InternFromString("dst_blocks");
@@ -103,6 +109,13 @@ static HostPlan pack_chunks(const py::iterable& chunks, uint32_t tile_tokens, ui
   static PyObject* const kPad = PyUnicode_InternFromString("pad_tail");
   PlanPacker pk{tile_tokens, dst_ntpb, {}, {}};
   for (const py::handle c : chunks) {
+    if (!plain.is_none() && reinterpret_cast<PyObject*>(Py_TYPE(c.ptr())) != plain.ptr()) {
+      const py::object tuple = c.attr("as_tuple")();
+      py::detail::make_caster<ReqTuple> req;
+      if (!req.load(tuple, true)) throw py::type_error("kvt_pack_chunks: not a request's tuple");
+      add_tuple(pk, py::detail::cast_op<ReqTuple>(std::move(req)));
+      continue;
+    }
     auto attr = [&c](PyObject* name) {
       py::object o = py::reinterpret_steal<py::object>(PyObject_GetAttr(c.ptr(), name));
       if (!o) throw py::error_already_set();
@@ -186,7 +199,7 @@ void bind_kernels(py::module_& m) {
         if (!p.blob.empty()) check_cuda(kvt_copy_now(dst, p.blob.data(), p.blob.size(), reinterpret_cast<void*>(after)), "kvt_copy_now");
       }, py::arg("dst"), py::arg("after"), py::call_guard<py::gil_scoped_release>(),
            "The plan at a device address, behind the event `after`, complete on return and outside of any capture.");
-  m.def("kvt_pack_chunks", &pack_chunks, py::arg("chunks"), py::arg("tile_tokens"), py::arg("dst_ntpb"));
+  m.def("kvt_pack_chunks", &pack_chunks, py::arg("chunks"), py::arg("tile_tokens"), py::arg("dst_ntpb"), py::arg("plain") = py::none());
   m.def("kvt_stream_capturing", [](uint64_t stream) { return kvt_stream_capturing(reinterpret_cast<void*>(stream)) != 0; });
 
   m.def("kvt_req_tiles", &kvt_req_tiles);

@@ -132,7 +132,7 @@ class DevicePlan:
     def __init__(self, chunks: Sequence[ReqChunk], tile_tokens: int, dst_ntpb: int, device, stream=None,
                  pinned: Optional[torch.Tensor] = None, room: Optional[PlanRoom] = None):
         K = _ops()
-        self._host = host = K.kvt_pack_chunks(chunks, tile_tokens, dst_ntpb)
+        self._host = host = K.kvt_pack_chunks(chunks, tile_tokens, dst_ntpb, ReqChunk)
         self.n_reqs, self.total_tiles, self.pool_offset, self.nbytes = host.n_reqs, host.total_tiles, host.pool_offset, host.nbytes
         self.pinned, self.device = pinned, device
         self._dev: Optional[torch.Tensor] = None
