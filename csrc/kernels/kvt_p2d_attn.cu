@@ -35,6 +35,7 @@
 #include <string.h>
 
 #include "kvt_kernels.h"
+#include "smem_grant.h"
 
 namespace {
 
@@ -1144,18 +1145,15 @@ bool quant_staged(const KvtAttnLaunch& a) {
   return stage_env > 0 || (stage_env < 0 && a.dst_remote != 0);
 }
 
-// More than 48 KiB of shared memory, the kernel's own arrays (at most 1 KiB) included, take an opt-in, which is per device and
-// sticky: asked for once per device, and again only for a larger size.
+// More than 48 KiB of shared memory, the kernel's own arrays (at most 1 KiB) included, take an opt-in.
 template <typename KERNEL>
-cudaError_t opt_in(KERNEL kern, size_t smem, std::atomic<size_t> (&granted)[kMaxDevices]) {
+cudaError_t opt_in(KERNEL kern, size_t smem, SmemGrant& grant) {
   if (smem <= 47 * 1024) return cudaSuccess;
   int dev = 0;
   cudaGetDevice(&dev);
-  std::atomic<size_t>* slot = dev >= 0 && dev < kMaxDevices ? &granted[dev] : nullptr;
-  if (slot != nullptr && slot->load(std::memory_order_relaxed) >= smem) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess && slot != nullptr) slot->store(smem, std::memory_order_relaxed);
-  return e;
+  return (cudaError_t)grant.ask(dev, smem, [kern](size_t bytes) {
+    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  });
 }
 
 // The plan as a parameter of the launch.
@@ -1186,8 +1184,8 @@ cudaError_t launch_expand_as(const KvtAttnLaunch& a, int grid_ctas, int sms, uin
   const size_t smem = stages * stage_bytes;
   const auto go = [&](auto in_launch) {
     constexpr bool kIn = decltype(in_launch)::value;
-    static std::atomic<size_t> granted[kMaxDevices];
-    const cudaError_t e = opt_in(kvt_p2d_expand_kernel<SHAPE, kIn>, smem, granted);
+    static SmemGrant grant;
+    const cudaError_t e = opt_in(kvt_p2d_expand_kernel<SHAPE, kIn>, smem, grant);
     if (e != cudaSuccess) return e;
     kvt_p2d_expand_kernel<SHAPE, kIn><<<(int)grid, 32u * (1u + SHAPE::WARPS), smem, stream>>>(
         a, (uint32_t)stages, (uint32_t)tile_bytes, (uint32_t)stage_bytes, plan_param<kIn>(a));
@@ -1209,8 +1207,8 @@ template <int MODE, bool USE_TMA, bool IN_LAUNCH>
 cudaError_t launch_as(const KvtAttnLaunch& a, int grid, int threads, uint32_t stages, uint32_t tile_bytes, size_t smem,
                       uint32_t warp_tiles, cudaStream_t stream) {
   auto kern = kvt_p2d_attn_kernel<MODE, USE_TMA, IN_LAUNCH>;
-  static std::atomic<size_t> granted[kMaxDevices];
-  const cudaError_t e = opt_in(kern, smem, granted);
+  static SmemGrant grant;
+  const cudaError_t e = opt_in(kern, smem, grant);
   if (e != cudaSuccess) return e;
   kern<<<grid, threads, smem, stream>>>(a, stages, tile_bytes, warp_tiles, plan_param<IN_LAUNCH>(a));
   return cudaGetLastError();

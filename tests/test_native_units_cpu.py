@@ -1,0 +1,48 @@
+"""Native pieces that need no GPU, compiled on their own with fakes of the driver's calls."""
+import shutil
+import subprocess
+import textwrap
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "csrc"
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+
+
+def _run(tmp_path, source):
+    (tmp_path / "t.cpp").write_text(textwrap.dedent(source))
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", f"-I{CSRC}", "-o", tmp_path / "t", tmp_path / "t.cpp"], check=True, timeout=120)
+    return subprocess.run([tmp_path / "t"], check=True, timeout=60, capture_output=True, text=True).stdout.split()
+
+
+def test_a_smaller_tile_never_takes_back_what_a_larger_one_was_granted(tmp_path):
+    """Two threads ask at once; the one that wants more is slow to note that it was granted."""
+    got = _run(tmp_path, """
+        #include "kernels/smem_grant.h"
+        #include <chrono>
+        #include <cstdio>
+        #include <thread>
+        int main() {
+          using namespace std::chrono_literals;
+          SmemGrant grant;
+          std::atomic<size_t> attribute{0};
+          std::atomic<int> calls{0};
+          auto set = [&](size_t bytes) {
+            ++calls;
+            attribute = bytes;
+            if (bytes > 49000) std::this_thread::sleep_for(300ms);
+            return 0;
+          };
+          std::thread large([&] { grant.ask(0, 50688, set); });
+          while (attribute == 0) std::this_thread::yield();
+          std::thread small([&] { grant.ask(0, 48576, set); });
+          large.join();
+          small.join();
+          const int refused = grant.ask(0, 50688, set);
+          std::printf("%zu %d %d ", attribute.load(), calls.load(), refused);
+          // another device, a failure that is not noted, and a device beyond the table
+          const int failed = grant.ask(1, 60000, [](size_t) { return 7; }), then = grant.ask(1, 60000, set), far = grant.ask(1000, 60000, set);
+          std::printf("%d %d %d %d", failed, then, far, calls.load());
+        }""")
+    assert got == ["50688", "1", "0", "7", "0", "0", "3"]
