@@ -88,7 +88,7 @@ DeviceStage::~DeviceStage() {
   if (done_event_ != nullptr) cudaEventDestroy(static_cast<cudaEvent_t>(done_event_));
   if (d_triples_ != nullptr) cudaFree(d_triples_);
   if (d_status_ != nullptr) cudaFree(d_status_);
-  if (d_staging_ != nullptr) cudaFree(d_staging_);
+  if (staging_.data() != nullptr) cudaFree(staging_.data());
 }
 
 void* DeviceStage::record_done() {
@@ -227,21 +227,20 @@ uint64_t DeviceStage::dense_source(const std::vector<Triple>& triples, uint64_t 
   return total < kStagingLeast || total > kStagingMax || first > src_cap || total > src_cap - first ? 0 : total;
 }
 
-void DeviceStage::reserve_staging(size_t bytes) {
-  bytes = std::min(bytes, kStagingMax);
-  if (bytes <= staging_cap_) return;
+bool DeviceStage::reserve_staging(size_t bytes) {
   cuda_check(cudaSetDevice(device_), "cudaSetDevice");
-  void* p = nullptr;
-  if (cudaMalloc(&p, bytes) != cudaSuccess) {      // no room: the lists go through the mapping
-    cudaGetLastError();
-    return;
-  }
-  if (d_staging_ != nullptr) {
-    cudaStreamSynchronize(static_cast<cudaStream_t>(stream_));
-    cudaFree(d_staging_);
-  }
-  d_staging_ = static_cast<char*>(p);
-  staging_cap_ = bytes;
+  return staging_.reserve(
+      std::min(bytes, kStagingMax),
+      [](size_t n) {
+        void* p = nullptr;
+        if (cudaMalloc(&p, n) == cudaSuccess) return p;
+        cudaGetLastError();      // no room: the lists go through the mapping
+        return static_cast<void*>(nullptr);
+      },
+      [this](void* smaller) {
+        cudaStreamSynchronize(static_cast<cudaStream_t>(stream_));
+        cudaFree(smaller);
+      });
 }
 
 // A copy engine brings host memory at 55.3 GB/s where the loads of the SMs reach 51.1, and beside SM stores in the other direction, as
@@ -257,18 +256,17 @@ void DeviceStage::enqueue_from_host(uint64_t src_base, uint64_t dst_base, const 
   kernel_lists_++;
   g_kernel_lists++;
   const uint64_t total = dense_source(triples, src_cap);
-  if (total != 0) reserve_staging(total);
-  if (total == 0 || staging_cap_ < total) {
+  if (total == 0 || !reserve_staging(total)) {
     launch_new(src_base, dst_base, triples.data(), triples.size(), src_cap, dst_cap, 0, HOST_SRC, false);
     return;
   }
   const uint64_t from = triples[0].src_off;
-  cuda_check(cudaMemcpyAsync(d_staging_, reinterpret_cast<const void*>(src_base + from), total, cudaMemcpyDefault,
+  cuda_check(cudaMemcpyAsync(staging_.data(), reinterpret_cast<const void*>(src_base + from), total, cudaMemcpyDefault,
                              static_cast<cudaStream_t>(stream_)),
              "cudaMemcpyAsync(staging)");
   std::vector<Triple> local(triples);
   for (Triple& t : local) t.src_off -= from;
-  launch_new(reinterpret_cast<uint64_t>(d_staging_), dst_base, local.data(), local.size(), total, dst_cap, 0, HOST_NONE, false);
+  launch_new(reinterpret_cast<uint64_t>(staging_.data()), dst_base, local.data(), local.size(), total, dst_cap, 0, HOST_NONE, false);
 }
 
 void DeviceStage::forget(size_t lists_total) {

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "kernels/kvt_kernels.h"
+#include "transport/staging_buffer.h"
 
 namespace kvx {
 
@@ -66,7 +67,7 @@ class DeviceStage {
   size_t keep(const std::vector<Triple>& triples);
   void enqueue_kept(uint64_t src_base, uint64_t dst_base, size_t place, const std::vector<Triple>& triples, uint64_t src_cap,
                     uint64_t dst_cap, int host_side, bool cast_bf16_e4m3);
-  void reserve_staging(size_t bytes);
+  bool reserve_staging(size_t bytes);      // false: it is not to be had
   static constexpr size_t kStagingLeast = 512u << 10, kStagingMax = 32u << 20;
   // A mark is a completion record in mapped host memory behind everything enqueued so far; at most kMarks are open, and they are
   // waited for in order.  wait_mark() returns when it has arrived and throws as sync() does; poll_mark() says whether it has.
@@ -113,8 +114,7 @@ class DeviceStage {
   KvtCompletion* d_marks_{nullptr};
   uint64_t marks_{0}, waited_{0};        // enqueued, waited for
   uint32_t polls_{0};
-  char* d_staging_{nullptr};
-  size_t staging_cap_{0};
+  StagingBuffer staging_;
   uint64_t memcpy_lists_{0};
   uint64_t kernel_lists_{0};
 };

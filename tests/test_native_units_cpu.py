@@ -46,3 +46,26 @@ def test_a_smaller_tile_never_takes_back_what_a_larger_one_was_granted(tmp_path)
           std::printf("%d %d %d %d", failed, then, far, calls.load());
         }""")
     assert got == ["50688", "1", "0", "7", "0", "0", "3"]
+
+
+def test_a_staging_buffer_that_cannot_be_had_is_not_asked_for_again(tmp_path):
+    """The GPU has 8 MiB left: 16 are refused once, 4 and then 8 are had, what is larger stays refused."""
+    got = _run(tmp_path, """
+        #include "transport/staging_buffer.h"
+        #include <cstdio>
+        #include <initializer_list>
+        int main() {
+          kvx::StagingBuffer b;
+          static char memory[2];
+          int asked = 0, given = 0, back = 0;
+          auto alloc = [&](size_t n) -> void* { ++asked; return n <= (8u << 20) ? &memory[given++] : nullptr; };
+          auto release = [&](void*) { ++back; };
+          auto step = [&](size_t mib) {
+            const bool ok = b.reserve(mib << 20, alloc, release);
+            std::printf("%d/%d ", static_cast<int>(ok), asked);
+          };
+          for (size_t mib : {16, 16, 32, 16, 4, 4, 16, 8, 2, 16}) step(mib);
+          std::printf("%d %d", given, back);
+          return b.data() == &memory[1] ? 0 : 1;
+        }""")
+    assert got == ["0/1", "0/1", "0/1", "0/1", "1/2", "1/2", "0/2", "1/3", "1/3", "0/3", "2", "1"]
