@@ -200,6 +200,7 @@ class KvClient {
   void share_layer_events() {
     if (barrier_ != nullptr) barrier_->share();
   }
+  bool layer_event_ready(uint32_t layer) { return barrier_ == nullptr || barrier_->ready(layer); }
   void record_event(uint64_t event, uint64_t stream) {
     if (barrier_ != nullptr) barrier_->record(event, stream);
     else cuda_check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "cudaEventRecord(layer)");
@@ -496,6 +497,7 @@ void bind_engine(py::module_& m) {
       .def("record_layer",
            [](KvClient& c, size_t stepid, uint64_t event, uint64_t stream) { c.record_layer(stepid, event, stream); })
       .def("share_layer_events", [](KvClient& c) { c.share_layer_events(); }, "As when a peer asks for the layer events.")
+      .def("layer_event_ready", &KvClient::layer_event_ready)
       .def("record_layer_event", [](KvClient& c, uint64_t event, uint64_t stream) { c.record_event(event, stream); })
       .def("flush_send", [](KvClient& c, size_t stepid) { c.get()->flush_send(stepid); })
       .def("drain", [](KvClient& c) { c.get()->drain(); }, py::call_guard<py::gil_scoped_release>())
@@ -607,6 +609,7 @@ void bind_engine(py::module_& m) {
   });
   m.def("notify_event_record", [](size_t stepid) { need_client()->notify_event_record(stepid); });
   m.def("record_layer", [](size_t stepid, uint64_t event, uint64_t stream) { need_kv_client().record_layer(stepid, event, stream); });
+  m.def("layer_event_ready", [](uint32_t layer) { return need_kv_client().layer_event_ready(layer); });
   m.def("record_layer_event", [](uint64_t event, uint64_t stream) { need_kv_client().record_event(event, stream); });
   m.def("flush_send", [](size_t stepid) { need_client()->flush_send(stepid); });
   m.def(

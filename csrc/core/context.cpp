@@ -41,6 +41,17 @@ void CudaEventBarrier::record(uint64_t event, uint64_t stream) {
   check(cudaEventRecord(reinterpret_cast<cudaEvent_t>(event), reinterpret_cast<cudaStream_t>(stream)), "cudaEventRecord(layer)");
 }
 
+bool CudaEventBarrier::ready(uint32_t layer) {
+  RTASSERT(layer < events_.size());
+  const cudaError_t e = cudaEventQuery(static_cast<cudaEvent_t>(event(layer)));
+  if (e == cudaErrorNotReady) {
+    cudaGetLastError();
+    return false;
+  }
+  check(e, "cudaEventQuery");
+  return true;
+}
+
 void CudaEventBarrier::wait(uint32_t layer) {
   RTASSERT(layer < events_.size());
   cudaError_t e = cudaEventSynchronize(static_cast<cudaEvent_t>(event(layer)));      // once shared, the plain ones are of earlier steps

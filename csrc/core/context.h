@@ -51,6 +51,8 @@ class CudaEventBarrier : public ICudaBarrier {
   }
   // From here on the peer events are the layers' events; what the plain ones stand for so far is carried over.
   void share() override;
+  // What the layer's latest record stands for has happened.
+  bool ready(uint32_t layer);
   // Engine thread: layer event `event` (its plain one) on `stream`.
   void record(uint64_t event, uint64_t stream);
 

@@ -348,7 +348,7 @@ class KVTransferClient:
             raise RuntimeError("KVTransferClient not inited")
         if self._cur_step_id is None:
             return
-        if self._events and not self._events[-1].query() and not self._async_sched_warned:
+        if self._events and not self._async_sched_warned and not self._call("layer_event_ready", self._num_layers - 1):
             self._async_sched_warned = True
             # The reference warns here because its step protocol cannot run ahead of the GPU.  Device-ordered
             # transports (NVLINK) order themselves after each layer's event, so this is only worth a note.
