@@ -95,7 +95,7 @@ struct HybridArgs {
   // the worker's cache as a member of an NVLink multicast group: multicast address per [layer][tensor], group size
   std::vector<std::vector<uint64_t>> mc_layers;
   uint32_t mc_size = 0;
-  std::vector<uint64_t> peer_events;     // client: interprocess events, one a layer, beside `events`
+  uint32_t peer_events = 0;              // client: 1: interprocess events beside `events` once a peer asks for them
 };
 
 void apply_hybrid(WorkerInfo* wi, const HybridArgs& h) {
@@ -179,7 +179,7 @@ class KvClient {
     if (!send_done_addr.empty()) ctx->worker_info_mutable()->ext["sdaddr"] = send_done_addr;
     if (!events.empty()) {
       RTASSERT(events.size() == layers.size());
-      auto barrier = std::make_unique<CudaEventBarrier>(events, h.peer_events);
+      auto barrier = std::make_unique<CudaEventBarrier>(events, h.peer_events != 0, device_id);
       barrier_ = barrier.get();
       ctx->set_cuda_barrier(std::move(barrier));
     }
@@ -199,6 +199,11 @@ class KvClient {
   }
   void share_layer_events() {
     if (barrier_ != nullptr) barrier_->share();
+  }
+  void wait_layer_event(uint32_t layer, uint64_t stream) {
+    if (barrier_ != nullptr)
+      cuda_check(cudaStreamWaitEvent(reinterpret_cast<cudaStream_t>(stream), static_cast<cudaEvent_t>(barrier_->event(layer)), 0),
+                 "cudaStreamWaitEvent(layer)");
   }
   bool layer_event_ready(uint32_t layer) { return barrier_ == nullptr || barrier_->ready(layer); }
   void record_event(uint64_t event, uint64_t stream) {
@@ -497,6 +502,7 @@ void bind_engine(py::module_& m) {
       .def("record_layer",
            [](KvClient& c, size_t stepid, uint64_t event, uint64_t stream) { c.record_layer(stepid, event, stream); })
       .def("share_layer_events", [](KvClient& c) { c.share_layer_events(); }, "As when a peer asks for the layer events.")
+      .def("wait_layer_event", &KvClient::wait_layer_event)
       .def("layer_event_ready", &KvClient::layer_event_ready)
       .def("record_layer_event", [](KvClient& c, uint64_t event, uint64_t stream) { c.record_event(event, stream); })
       .def("flush_send", [](KvClient& c, size_t stepid) { c.get()->flush_send(stepid); })
@@ -609,6 +615,7 @@ void bind_engine(py::module_& m) {
   });
   m.def("notify_event_record", [](size_t stepid) { need_client()->notify_event_record(stepid); });
   m.def("record_layer", [](size_t stepid, uint64_t event, uint64_t stream) { need_kv_client().record_layer(stepid, event, stream); });
+  m.def("wait_layer_event", [](uint32_t layer, uint64_t stream) { need_kv_client().wait_layer_event(layer, stream); });
   m.def("layer_event_ready", [](uint32_t layer) { return need_kv_client().layer_event_ready(layer); });
   m.def("record_layer_event", [](uint64_t event, uint64_t stream) { need_kv_client().record_event(event, stream); });
   m.def("flush_send", [](size_t stepid) { need_client()->flush_send(stepid); });

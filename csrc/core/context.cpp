@@ -10,16 +10,41 @@ static void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw KVTransferException(ErrorKind::CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-CudaEventBarrier::CudaEventBarrier(std::vector<uint64_t> events, std::vector<uint64_t> peer_events)
-    : events_(std::move(events)), peer_events_(std::move(peer_events)) {
-  RTASSERT(peer_events_.empty() || peer_events_.size() == events_.size());
-  for (size_t l = 0; l < peer_events_.size(); ++l) peer_of_[events_[l]] = peer_events_[l];
+// The calling thread's current device is `device` for as long as this lives.
+struct OnDevice {
+  explicit OnDevice(int device) {
+    cudaGetDevice(&before);
+    if (device >= 0) cudaSetDevice(device);
+  }
+  ~OnDevice() { cudaSetDevice(before); }
+  int before{0};
+};
+
+CudaEventBarrier::~CudaEventBarrier() {
+  for (uint64_t e : peer_events_) cudaEventDestroy(reinterpret_cast<cudaEvent_t>(e));
+}
+
+bool CudaEventBarrier::make_peer_events() {
+  if (peer_events_.size() == events_.size()) return true;
+  for (size_t l = peer_events_.size(); l < events_.size(); ++l) {
+    cudaEvent_t e = nullptr;
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming | cudaEventInterprocess) != cudaSuccess) {
+      cudaGetLastError();
+      break;
+    }
+    peer_events_.push_back(reinterpret_cast<uint64_t>(e));
+    peer_of_[events_[l]] = peer_events_.back();
+  }
+  return peer_events_.size() == events_.size();
 }
 
 void CudaEventBarrier::share() {
-  if (peer_events_.empty()) return;
-  std::lock_guard<std::mutex> g(mu_);
+  if (!peers_ || shared_.load(std::memory_order_acquire)) return;
+  std::lock_guard<std::mutex> one(share_mu_);
   if (shared_.load(std::memory_order_relaxed)) return;
+  const OnDevice here(device_);
+  if (!make_peer_events()) return;     // the plain ones stay: a peer in another process sees that they have no handles
+  std::lock_guard<std::mutex> g(mu_);
   cudaStream_t s = nullptr;
   check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
   cudaError_t e = cudaSuccess;

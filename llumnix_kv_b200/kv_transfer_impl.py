@@ -190,6 +190,14 @@ def _hybrid_kwargs(num_kv_heads, num_gdn_layers, indexer_blk_ntpb, hybrid_indexe
         ple_conv_channel_dims=list(ple_conv_channel_dims or []))
 
 
+class _LayerEvent:
+    def __init__(self, client, layer):
+        self._client, self._layer = client, layer
+
+    def wait(self, stream):     # torch.cuda.Stream.wait_event(self)
+        self._client._call("wait_layer_event", self._layer, stream.cuda_stream)
+
+
 class KVTransferClient:
     """Sender side: submit request chunks, open a step, record one event per layer, flush."""
 
@@ -219,8 +227,8 @@ class KVTransferClient:
                             gdn_conv_channel_dims, kda_conv_dim_first, hybrid_attn_token_size, kda_page_stride,
                             attn_pack_size, num_ple_layers, ple_block_group, ple_conv_elem_size,
                             ple_conv_state_shape, ple_conv_channel_dims)
-        if self._peer_events:
-            kw["peer_events"] = [ev.cuda_event for ev in self._peer_events]
+        if self._events:
+            kw["peer_events"] = 1
         if mc_layers is not None and mc_size > 1:
             mc = [[int(a)] if isinstance(a, int) else [int(x) for x in a] for a in mc_layers]
             assert len(mc) == len(layer_addrs) and all(len(a) == len(b) for a, b in zip(mc, layer_addrs))
@@ -254,17 +262,22 @@ class KVTransferClient:
     def _init_events(self):
         if self._device_id >= 0:
             with torch.cuda.device(self._device_id):
-                # a decode worker that pulls this cache orders its streams after the interprocess ones (CUDA IPC event
-                # handles), so nobody's host waits for the forward pass; until there is one the plain ones serve
+                # a decode worker that pulls this cache orders its streams after interprocess events (CUDA IPC event
+                # handles), so nobody's host waits for the forward pass; the engine makes those when one asks, and until
+                # then these serve
                 self._events = [torch.cuda.Event() for _ in range(self._num_layers)]
-                self._peer_events = [torch.cuda.Event(interprocess=True) for _ in range(self._num_layers)]
                 stream = torch.cuda.current_stream()      # looked up once, not for each event
-                for ev in self._events + self._peer_events:
+                for ev in self._events:
                     ev.record(stream)
             self._event_addrs = [ev.cuda_event for ev in self._events]
         else:
-            self._events, self._peer_events = [], []
+            self._events = []
             self._event_addrs = []
+
+    @property
+    def _peer_events(self):
+        """Per layer, what a stream of this process waits for: the event that serves now."""
+        return [_LayerEvent(self, layer) for layer in range(len(self._events))]
 
     # ---- engine calls ---------------------------------------------------------------------
     def _call(self, name, *args):

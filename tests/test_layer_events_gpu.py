@@ -46,3 +46,37 @@ def test_a_flush_ahead_of_the_last_layer_is_noted(pair, caplog, shared, late):
         cli.flush_send_step()
     assert any("before the last layer event" in r.message for r in caplog.records) == late
     assert cli.wait_inflight(0, 30.0) and not cli.failed_batches()
+
+
+def test_interprocess_events_are_made_when_a_peer_asks(ops, monkeypatch):
+    real, made = torch.cuda.Event, []
+
+    def event(*a, **kw):
+        made.append(bool(kw.get("interprocess", False)))
+        return real(*a, **kw)
+
+    monkeypatch.setattr(torch.cuda, "Event", event)
+    lay = AttnLayout(CacheShape.FLASH, 8, 16, 8, 128, 2)
+    src = [lay.alloc(DEV) for _ in range(LAYERS)]
+    cli = KVTransferClient("P|0|1", 1, 0, 0, lay.block_bytes, lay.token_bytes, "fake://", src, [PT.NVLINK],
+                           num_kv_heads=8, cache_shape=int(CacheShape.FLASH))
+    try:
+        assert made == [False] * LAYERS
+        s, seen, big = torch.cuda.Stream(), torch.zeros_like(src[0]), torch.empty(1 << 30, dtype=torch.uint8, device=DEV)
+        torch.cuda.synchronize()
+        for v in (1, 2, 3):
+            for _ in range(20):
+                big.fill_(v)
+            src[-1].fill_(v)
+            cli._c.record_layer_event(cli._event_addrs[-1], torch.cuda.current_stream().cuda_stream)
+            if v == 2:
+                cli._c.share_layer_events()     # carries over what is pending
+            s.wait_event(cli._peer_events[-1])
+            with torch.cuda.stream(s):
+                seen.copy_(src[-1], non_blocking=True)
+            s.synchronize()
+            assert int(seen.min()) == int(seen.max()) == v
+            assert cli._c.layer_event_ready(LAYERS - 1)
+    finally:
+        cli.drain()
+        del cli
