@@ -132,8 +132,10 @@ class PinnedKVStore:
                 self.uses_tma = tma
                 self._save_xfer = AttnTransfer(engine_layout, self.page, eng_ptrs, page_ptrs, self.device,
                                                mode=MODE_BF16_TO_MXFP8 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2)
+                self._status = self._save_xfer.status      # of every transfer of this store: one read of the device tells
                 self._load_xfer = AttnTransfer(self.page, engine_layout, page_ptrs, eng_ptrs, self.device,
-                                               mode=MODE_MXFP8_TO_BF16 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2)
+                                               mode=MODE_MXFP8_TO_BF16 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2,
+                                               status=self._status)
                 self.uses_tma = tma and self._save_xfer.use_tma and self._load_xfer.use_tma
                 if not tma:
                     self._init_staging(engine_layout, eng_ptrs, n_slots)
@@ -154,9 +156,9 @@ class PinnedKVStore:
             self._staging.record_stream(s)
         ptrs = [self._staging.data_ptr() + i * self.page_bytes for i in range(self.num_layers)]
         self._stage_save = AttnTransfer(engine_layout, page, eng_ptrs, ptrs, self.device,
-                                        mode=MODE_BF16_TO_MXFP8 if self.fp8 else MODE_COPY)
+                                        mode=MODE_BF16_TO_MXFP8 if self.fp8 else MODE_COPY, status=self._status)
         self._stage_load = AttnTransfer(page, engine_layout, ptrs, eng_ptrs, self.device,
-                                        mode=MODE_MXFP8_TO_BF16 if self.fp8 else MODE_COPY)
+                                        mode=MODE_MXFP8_TO_BF16 if self.fp8 else MODE_COPY, status=self._status)
         self._stage_grid = int(os.environ.get("BLLM_KVSTORE_CTAS", "0"))
         # per half: the kernel is through with it, the copy engine is
         self._kernel_done = [torch.cuda.Event() for _ in range(2)]
@@ -310,11 +312,10 @@ class PinnedKVStore:
         return self._move(False, layer_begin, layer_end, blocks, slots, after)
 
     def check_status(self) -> None:
-        for x in (self._save_xfer, self._load_xfer, self._stage_save, self._stage_load):
-            if x is not None:
-                code, detail = x.check_status()
-                if code != 0:
-                    raise RuntimeError(f"kv store transfer kernel reported status {code} (detail {detail})")
+        if self._save_xfer is not None:
+            code, detail = self._save_xfer.check_status()
+            if code != 0:
+                raise RuntimeError(f"kv store transfer kernel reported status {code} (detail {detail})")
 
     def stats(self) -> dict:
         return dict(self.kv.stats())

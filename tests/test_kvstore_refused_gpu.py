@@ -4,6 +4,7 @@ import torch
 
 from llumnix_kv_b200.kvstore import PinnedKVStore
 from llumnix_kv_b200.ops.layouts import AttnLayout, CacheShape
+from llumnix_kv_b200.ops.p2d_attn import AttnTransfer, ReqChunk
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -39,3 +40,27 @@ def test_a_refused_block_leaves_its_slot_alone(ops, fp8, at, bad):
     finally:
         st.close()
         ops.KvStore.unlink(name)
+
+
+def test_one_read_tells_about_all_transfers_of_a_store(ops, monkeypatch):
+    lay = AttnLayout(CacheShape.FLASH, N, 16, 8, 128, 2)
+    src = [lay.alloc(DEV, "normal", seed=i) for i in range(LAYERS)]
+    st = PinnedKVStore("kvx_status", lay, src, 0, 1, N, create=True)
+    try:
+        reads, look = [], AttnTransfer.check_status
+        monkeypatch.setattr(AttnTransfer, "check_status", lambda x: reads.append(x) or look(x))
+        st.check_status()
+        assert len(reads) == 1
+        for x in (st._save_xfer, st._load_xfer, st._stage_save, st._stage_load):
+            bad, good = [x.src_layout.num_blocks], [0]
+            x.launch(x.plan([ReqChunk(bad, good, 0, 16)], stream=st.stream), stream=st.stream)
+            st.stream.synchronize()
+            with pytest.raises(RuntimeError, match="status"):
+                st.check_status()
+            x.status.zero_()
+            torch.cuda.synchronize()
+            st.check_status()
+        assert len(reads) == 9
+    finally:
+        st.close()
+        ops.KvStore.unlink("kvx_status")
