@@ -1,0 +1,36 @@
+// Looking for a batch's completion record on the thread that sent it.
+#pragma once
+#include <atomic>
+
+namespace kvx {
+
+// One thread of a process at a time: whoever looks does not sleep, and with many targets as many sender threads would keep as many
+// cores from the engine's own threads.  The others hand their records to the completion poller, one thread for all.  CPU of the
+// sender threads a step of 16 layers and 900 us, 12 targets: 2330 us with a look by each, 1260 this way,
+// the step as long; 4 targets 680 and 400, one 162 both ways.
+class OwnLook {
+ public:
+  OwnLook() : mine_(!taken().exchange(true, std::memory_order_acquire)) {}
+  ~OwnLook() {
+    if (mine_) taken().store(false, std::memory_order_release);
+  }
+  OwnLook(const OwnLook&) = delete;
+  explicit operator bool() const { return mine_; }
+  // Between two looks: leaves the core's other thread and the memory bus alone for a moment.
+  static void pause() {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#elif defined(__aarch64__)
+    asm volatile("yield");
+#endif
+  }
+
+ private:
+  static std::atomic<bool>& taken() {
+    static std::atomic<bool> t{false};
+    return t;
+  }
+  const bool mine_;
+};
+
+}  // namespace kvx

@@ -10,6 +10,7 @@
 #include "core/completion.h"
 #include "core/envcfg.h"
 #include "core/fault_inject.h"
+#include "core/own_look.h"
 #include "plan/device_plan.h"
 #include "plan/planner.h"
 #include "transport/verify.h"
@@ -425,13 +426,16 @@ struct KvSendStub::Impl {
     }
     // A batch that is all this stub has on the device, with nothing waiting for this thread: look for its record here for as long as
     // a short one takes.  The poller's thread would have to be woken first (10 us).  A batch whose end is reported to a scheduler,
-    // or checked, is left to the poller: the answer would hold up the next batch here.
+    // or checked, is left to the poller: the answer would hold up the next batch here.  So is one that ends while another thread looks.
     if (async && completing.load(std::memory_order_acquire) == 0 && check_ctx == nullptr && (pb.finished_req.empty() || !notifier.enabled())) {
       const Timepoint until = SteadyClock::now() + std::chrono::microseconds(100);
       PollResult r = PollResult::PENDING;
       try {
-        while (r == PollResult::PENDING && !ThreadPool::others_wait() && SteadyClock::now() < until)
+        const OwnLook look;
+        while (look && r == PollResult::PENDING && !ThreadPool::others_wait() && SteadyClock::now() < until) {
           r = pb.ch->poll_completion(pb.ticket, pb.flush_out);
+          if (r == PollResult::PENDING) OwnLook::pause();
+        }
       } catch (const std::exception& ex) {
         LOG(ERROR) << "completion poll failed: " << ex.what();
         r = PollResult::FAILED;

@@ -69,3 +69,39 @@ def test_a_staging_buffer_that_cannot_be_had_is_not_asked_for_again(tmp_path):
           return b.data() == &memory[1] ? 0 : 1;
         }""")
     assert got == ["0/1", "0/1", "0/1", "0/1", "1/2", "1/2", "0/2", "1/3", "1/3", "0/3", "2", "1"]
+
+
+def test_one_thread_at_a_time_looks_for_its_record(tmp_path):
+    got = _run(tmp_path, """
+        #include "core/own_look.h"
+        #include <cstdio>
+        #include <thread>
+        #include <vector>
+        using kvx::OwnLook;
+        int main() {
+          bool other = true, second = false;
+          {
+            OwnLook mine;
+            std::thread([&] { OwnLook l; other = static_cast<bool>(l); }).join();
+            OwnLook again;      // one that did not get it gives nothing back
+            std::printf("%d %d %d ", static_cast<bool>(mine), other, static_cast<bool>(again));
+          }
+          std::thread([&] { OwnLook l; second = static_cast<bool>(l); }).join();
+          std::atomic<int> inside{0}, most{0}, had{0};
+          std::vector<std::thread> all;
+          for (int t = 0; t < 8; ++t)
+            all.emplace_back([&] {
+              for (int i = 0; i < 2000; ++i) {
+                OwnLook l;
+                if (!l) continue;
+                const int n = ++inside;
+                if (n > most) most = n;
+                ++had;
+                OwnLook::pause();
+                --inside;
+              }
+            });
+          for (auto& t : all) t.join();
+          std::printf("%d %d %d", second, most.load(), had.load() > 0);
+        }""")
+    assert got == ["1", "0", "0", "1", "1", "1"]
