@@ -2,6 +2,7 @@
 
 #include <arpa/inet.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -106,6 +107,7 @@ size_t env_copy_memcpy_max_blocks() { return (size_t)posint("BLLM_KVTRANS_COPY_M
 size_t env_copy_memcpy_threshold_bytes() { return (size_t)posint("BLLM_KVTRANS_COPY_MEMCPY_BLOCK_THRESHOLD_BYTES", 256 * 1024); }
 bool env_device_timestamps() { return anyint("BLLM_KVTRANS_DEVICE_TIMESTAMPS", 0) != 0; }
 int env_copy_path() { return (int)anyint("BLLM_KVTRANS_COPY_PATH", 0); }
+size_t env_staging_bytes() { return (size_t)std::clamp<long>(anyint("BLLM_KVTRANS_STAGING_MB", 32), 0, 1 << 20) << 20; }
 
 double env_kernel_copy_sm_usage() noexcept {
   std::lock_guard<std::mutex> g(g_mu);

@@ -77,6 +77,9 @@ bool env_copy_profile_enable();
 size_t env_copy_memcpy_max_blocks();
 size_t env_copy_memcpy_threshold_bytes();
 int env_copy_path();
+// Most GPU memory that the receiving end of a host-staged connection takes for staging a layer's frame (0: none, frames are
+// read through the mapping).  It comes from cudaMalloc, beside what torch's allocator holds.
+size_t env_staging_bytes();
 // NVLink channel: stamp the GPU timer at the start and the end of every batch and report DeviceUs in the flush line.
 bool env_device_timestamps();
 // How long a batch of a device transport may take to deliver its completion record before it is failed

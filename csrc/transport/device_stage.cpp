@@ -224,13 +224,14 @@ uint64_t DeviceStage::dense_source(const std::vector<Triple>& triples, uint64_t 
     total += t.len;
   }
   const uint64_t first = triples[0].src_off;
-  return total < kStagingLeast || total > kStagingMax || first > src_cap || total > src_cap - first ? 0 : total;
+  return total < kStagingLeast || total > env_staging_bytes() || first > src_cap || total > src_cap - first ? 0 : total;
 }
 
 bool DeviceStage::reserve_staging(size_t bytes) {
+  if (bytes > env_staging_bytes()) return false;     // a blob is staged whole or not at all
   cuda_check(cudaSetDevice(device_), "cudaSetDevice");
   return staging_.reserve(
-      std::min(bytes, kStagingMax),
+      bytes,
       [](size_t n) {
         void* p = nullptr;
         if (cudaMalloc(&p, n) == cudaSuccess) return p;

@@ -58,7 +58,7 @@ class DeviceStage {
                uint64_t dst_cap, int grid_ctas = 0, int host_side = HOST_NONE, bool cast_bf16_e4m3 = false);
   uint64_t memcpy_lists() const { return memcpy_lists_; }   // lists that went to the copy engines
   uint64_t kernel_lists() const { return kernel_lists_; }
-  // Pinned host memory -> scattered runs.  A list whose source is one dense run of kStagingLeast to kStagingMax bytes crosses PCIe as one
+  // Pinned host memory -> scattered runs.  A list whose source is one dense run of kStagingLeast to env_staging_bytes() bytes crosses PCIe as one
   // copy of the copy engine into this stage's own buffer, from where the kernel scatters it; any other is read through the mapping.
   void enqueue_from_host(uint64_t src_base, uint64_t dst_base, const std::vector<Triple>& triples, uint64_t src_cap, uint64_t dst_cap);
   // Lists that several launches use: uploaded once by keep() (after forget(), with nothing enqueued still running; it returns the
@@ -68,7 +68,7 @@ class DeviceStage {
   void enqueue_kept(uint64_t src_base, uint64_t dst_base, size_t place, const std::vector<Triple>& triples, uint64_t src_cap,
                     uint64_t dst_cap, int host_side, bool cast_bf16_e4m3);
   bool reserve_staging(size_t bytes);      // false: it is not to be had
-  static constexpr size_t kStagingLeast = 512u << 10, kStagingMax = 32u << 20;
+  static constexpr size_t kStagingLeast = 512u << 10;
   // A mark is a completion record in mapped host memory behind everything enqueued so far; at most kMarks are open, and they are
   // waited for in order.  wait_mark() returns when it has arrived and throws as sync() does; poll_mark() says whether it has.
   static constexpr size_t kMarks = 8;

@@ -137,7 +137,8 @@ class PinnedKVStore:
                                                mode=MODE_MXFP8_TO_BF16 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2,
                                                status=self._status)
                 self.uses_tma = tma and self._save_xfer.use_tma and self._load_xfer.use_tma
-                if not tma:
+                # BLLM_KVSTORE_STAGING=0: no buffer on the GPU (32 MiB a store, out of torch's allocator), every move through the mapping
+                if not tma and os.environ.get("BLLM_KVSTORE_STAGING", "1") not in ("0", ""):
                     self._init_staging(engine_layout, eng_ptrs, n_slots)
 
     def _init_staging(self, engine_layout: AttnLayout, eng_ptrs: List[int], n_slots: int) -> None:
