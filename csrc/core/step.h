@@ -23,7 +23,7 @@ class Step {
  public:
   const size_t step_idx;
   const Timepoint start_send_ts = SteadyClock::now();
-  std::vector<int64_t> sub_queue_time_us;  // written by the target-manager thread
+  std::vector<int64_t> sub_queue_time_us;  // written by whoever submits: the engine thread, or the target manager's under its lock
   Timepoint flush_send_ts;                 // written by the engine thread
   Timepoint wait_layers_start_ts;          // written by the wait-layers thread
   Timepoint wait_layers_end_ts;
