@@ -194,6 +194,8 @@ void bind_kernels(py::module_& m) {
       .def_readonly("total_tiles", &HostPlan::total_tiles)
       .def_readonly("pool_offset", &HostPlan::pool_offset)
       .def_property_readonly("nbytes", [](const HostPlan& p) { return p.blob.size(); })
+      .def_property_readonly("sizes", [](const HostPlan& p) { return py::make_tuple(p.n_reqs, p.total_tiles, p.pool_offset, p.blob.size()); },
+                             "(n_reqs, total_tiles, pool_offset, nbytes) in one look: four cost a plan 0.15 us more")
       .def_property_readonly("blob", [](const HostPlan& p) { return py::bytes(p.blob); })
       .def("copy_to_device", [](const HostPlan& p, uint64_t dst, uint64_t after) {
         if (!p.blob.empty()) check_cuda(kvt_copy_now(dst, p.blob.data(), p.blob.size(), reinterpret_cast<void*>(after)), "kvt_copy_now");

@@ -133,14 +133,14 @@ class DevicePlan:
                  pinned: Optional[torch.Tensor] = None, room: Optional[PlanRoom] = None):
         K = _ops()
         self._host = host = K.kvt_pack_chunks(chunks, tile_tokens, dst_ntpb, ReqChunk)
-        self.n_reqs, self.total_tiles, self.pool_offset, self.nbytes = host.n_reqs, host.total_tiles, host.pool_offset, host.nbytes
+        self.n_reqs, self.total_tiles, self.pool_offset, self.nbytes = host.sizes
         self.pinned, self.device = pinned, device
         self._dev: Optional[torch.Tensor] = None
-        n = max(self.nbytes, 16)
-        if room is not None and pinned is None and self.nbytes <= K.KVT_PLAN_IN_LAUNCH:
+        if room is not None and pinned is None and self.nbytes <= room.place_bytes:
             self._place = room.take(stream)
             if self._place is not None:
                 return
+        n = max(self.nbytes, 16)
         if pinned is None or pinned.numel() < n:
             self.pinned = pinned = torch.empty(n, dtype=torch.uint8, pin_memory=torch.cuda.is_available())
         if self.nbytes:
