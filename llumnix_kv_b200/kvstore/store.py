@@ -130,12 +130,12 @@ class PinnedKVStore:
                 # instead of the SIMT warps; bf16 pages only (the fp8 pages are written by the quantiser)
                 tma = os.environ.get("BLLM_KVSTORE_TMA", "0") not in ("0", "") and not fp8
                 self.uses_tma = tma
-                self._save_xfer = AttnTransfer(engine_layout, self.page, eng_ptrs, page_ptrs, self.device,
-                                               mode=MODE_BF16_TO_MXFP8 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2)
-                self._status = self._save_xfer.status      # of every transfer of this store: one read of the device tells
+                with torch.cuda.stream(self.stream):    # where its plans' memory is used, so that no move has to get some first
+                    self._save_xfer = AttnTransfer(engine_layout, self.page, eng_ptrs, page_ptrs, self.device,
+                                                   mode=MODE_BF16_TO_MXFP8 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2)
                 self._load_xfer = AttnTransfer(self.page, engine_layout, page_ptrs, eng_ptrs, self.device,
                                                mode=MODE_MXFP8_TO_BF16 if fp8 else MODE_COPY, use_tma=tma, simt_tile=2,
-                                               status=self._status)
+                                               beside=self._save_xfer)
                 self.uses_tma = tma and self._save_xfer.use_tma and self._load_xfer.use_tma
                 # BLLM_KVSTORE_STAGING=0: no buffer on the GPU (32 MiB a store, out of torch's allocator), every move through the mapping
                 if not tma and os.environ.get("BLLM_KVSTORE_STAGING", "1") not in ("0", ""):
@@ -157,9 +157,9 @@ class PinnedKVStore:
             self._staging.record_stream(s)
         ptrs = [self._staging.data_ptr() + i * self.page_bytes for i in range(self.num_layers)]
         self._stage_save = AttnTransfer(engine_layout, page, eng_ptrs, ptrs, self.device,
-                                        mode=MODE_BF16_TO_MXFP8 if self.fp8 else MODE_COPY, status=self._status)
+                                        mode=MODE_BF16_TO_MXFP8 if self.fp8 else MODE_COPY, beside=self._save_xfer)
         self._stage_load = AttnTransfer(page, engine_layout, ptrs, eng_ptrs, self.device,
-                                        mode=MODE_MXFP8_TO_BF16 if self.fp8 else MODE_COPY, status=self._status)
+                                        mode=MODE_MXFP8_TO_BF16 if self.fp8 else MODE_COPY, beside=self._save_xfer)
         self._stage_grid = int(os.environ.get("BLLM_KVSTORE_CTAS", "0"))
         # per half: the kernel is through with it, the copy engine is
         self._kernel_done = [torch.cuda.Event() for _ in range(2)]
@@ -313,7 +313,7 @@ class PinnedKVStore:
         return self._move(False, layer_begin, layer_end, blocks, slots, after)
 
     def check_status(self) -> None:
-        if self._save_xfer is not None:
+        if self._save_xfer is not None:      # its status is that of all the store's transfers
             code, detail = self._save_xfer.check_status()
             if code != 0:
                 raise RuntimeError(f"kv store transfer kernel reported status {code} (detail {detail})")

@@ -180,7 +180,7 @@ class AttnTransfer:
                  dst_ptrs: Sequence[int], device, head_map: Optional[HeadMap] = None, mode: int = MODE_COPY,
                  tile_tokens: Optional[int] = None, use_tma: bool = True, simt_tile: int = 0,
                  dst_remote: bool = False, tile_order: Optional[int] = None, store_form: Optional[int] = None,
-                 tma_stages: int = 0, cache_hint: int = 0, status: Optional[torch.Tensor] = None):
+                 tma_stages: int = 0, cache_hint: int = 0, beside: Optional["AttnTransfer"] = None):
         K = _ops()
         assert len(src_ptrs) == len(dst_ptrs)
         self.K = K
@@ -197,11 +197,11 @@ class AttnTransfer:
         self.tile_tokens = tile_tokens or math.gcd(src_layout.ntpb, dst_layout.ntpb)
         self.src_layers = torch.tensor(list(src_ptrs), dtype=torch.int64, device=self.device)
         self.dst_layers = torch.tensor(list(dst_ptrs), dtype=torch.int64, device=self.device)
-        # status[0] error code, status[1] detail, status[2] done counter (kept apart from flags); transfers that launch on one
-        # stream may share it, and one look then tells about all of them
-        self.status = torch.zeros(4, dtype=torch.int32, device=self.device) if status is None else status
-        self._room = None
-        if self.device.type == "cuda":
+        # status[0] error code, status[1] detail, status[2] done counter (kept apart from flags).  `beside`: a transfer that
+        # launches on the same stream and shares its own, so that one look tells about both, and its plans' memory
+        self.status = torch.zeros(4, dtype=torch.int32, device=self.device) if beside is None else beside.status
+        self._room = None if beside is None else beside._room
+        if self._room is None and self.device.type == "cuda":
             self._room = PlanRoom(self.device, K.KVT_PLAN_IN_LAUNCH)
             self._room.take()       # the first slab, so that no plan waits for it
         self.src_maps = self.dst_maps = None

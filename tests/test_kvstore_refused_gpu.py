@@ -64,3 +64,22 @@ def test_one_read_tells_about_all_transfers_of_a_store(ops, monkeypatch):
     finally:
         st.close()
         ops.KvStore.unlink("kvx_status")
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_a_first_move_finds_its_plans_memory_at_hand(ops, fp8):
+    """A place on the store's stream is there before the first plan asks: getting memory from the driver took up to 10 ms of that move."""
+    lay = AttnLayout(CacheShape.FLASH, N, 16, 8, 128, 2)
+    src = [lay.alloc(DEV, "normal", seed=i) for i in range(LAYERS)]
+    st = PinnedKVStore("kvx_first_%d" % fp8, lay, src, 0, 1, N, create=True, fp8=fp8)
+    try:
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        events = [f(*at, list(range(n)), list(range(n))) for f in (st.save_layers, st.load_layers) for at in ((0, LAYERS), (1, 2)) for n in (N, 5)]
+        assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+        for e in events:
+            e.synchronize()
+        st.check_status()
+    finally:
+        st.close()
+        ops.KvStore.unlink("kvx_first_%d" % fp8)
