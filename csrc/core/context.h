@@ -39,8 +39,8 @@ class NoCudaBarrier : public ICudaBarrier {
 };
 
 // One event a layer.  With `peers` the caller's events serve until another process asks for them, and interprocess ones that are made
-// then from there on: an interprocess event costs 1.2 us to record on the forward thread, a plain one 0.5, and a client
-// that nobody pulls from is made sooner without (32 layers: 81 us, the first time in a process 480).
+// then from there on: an interprocess event costs 1.2 us to record on the forward thread, a plain one 0.5, and a client that nobody
+// pulls from is made sooner without (32 layers: 400 us instead of 500).
 class CudaEventBarrier : public ICudaBarrier {
  public:
   explicit CudaEventBarrier(std::vector<uint64_t> events, bool peers = false, int device = -1)
@@ -61,7 +61,7 @@ class CudaEventBarrier : public ICudaBarrier {
 
  private:
   bool make_peer_events();
-  std::vector<uint64_t> events_, peer_events_;     // peer_events_: written once, before shared_ is set
+  std::vector<uint64_t> events_, peer_events_;     // peer_events_: written before shared_ is set, not after
   const bool peers_;
   const int device_;
   std::unordered_map<uint64_t, uint64_t> peer_of_;

@@ -6,8 +6,8 @@ namespace kvx {
 
 // One thread of a process at a time: whoever looks does not sleep, and with many targets as many sender threads would keep as many
 // cores from the engine's own threads.  The others hand their records to the completion poller, one thread for all.  CPU of the
-// sender threads a step of 16 layers and 900 us, 12 targets: 2330 us with a look by each, 1260 this way,
-// the step as long; 4 targets 680 and 400, one 162 both ways.
+// sender threads a step of 16 layers and 900 us, 12 targets: 2330 us with a look by each, 1260 this way, the step as long; 4 targets
+// 680 and 400, one 162 both ways.
 class OwnLook {
  public:
   OwnLook() : mine_(!taken().exchange(true, std::memory_order_acquire)) {}

@@ -66,7 +66,7 @@ __device__ __forceinline__ void set_status(uint32_t* status, uint32_t code, uint
 
 // Where the plan is.  A short one travels in the launch's parameters (IN_LAUNCH): its upload would be a copy in front of the
 // kernel and, from Python, a pinned buffer and a device tensor.  us a pass with an uploaded plan / this way, packing included: one
-// layer of 333 tokens 33.1 / 8.9, fp8 -> bf16 of 32 layers of 4003 tokens 147 / 137, 24 blocks to host memory 1034 / 999.
+// layer of 333 tokens 33.1 / 8.2, fp8 -> bf16 of 32 layers of 4003 tokens 147 / 137, 24 blocks to host memory 1034 / 999.
 // The lanes read it by generic addresses, coalesced as from memory: an index into the parameter space would be served lane by lane.
 template <bool IN_LAUNCH>
 struct PlanParam {};

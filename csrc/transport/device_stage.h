@@ -58,8 +58,9 @@ class DeviceStage {
                uint64_t dst_cap, int grid_ctas = 0, int host_side = HOST_NONE, bool cast_bf16_e4m3 = false);
   uint64_t memcpy_lists() const { return memcpy_lists_; }   // lists that went to the copy engines
   uint64_t kernel_lists() const { return kernel_lists_; }
-  // Pinned host memory -> scattered runs.  A list whose source is one dense run of kStagingLeast to env_staging_bytes() bytes crosses PCIe as one
-  // copy of the copy engine into this stage's own buffer, from where the kernel scatters it; any other is read through the mapping.
+  // Pinned host memory -> scattered runs.  A list whose source is one dense run of kStagingLeast to env_staging_bytes() bytes crosses
+  // PCIe as one copy of the copy engine into this stage's own buffer, from where the kernel scatters it; any other is read through the
+  // mapping.
   void enqueue_from_host(uint64_t src_base, uint64_t dst_base, const std::vector<Triple>& triples, uint64_t src_cap, uint64_t dst_cap);
   // Lists that several launches use: uploaded once by keep() (after forget(), with nothing enqueued still running; it returns the
   // list's place), then enqueued between whatever bases their offsets are meant for.  `triples` is the same list.

@@ -64,14 +64,14 @@ class HeadMap:
 
 
 class PlanRoom:
-    """Device memory for the short plans of one ``AttnTransfer``, should they ever be needed on the device.
+    """Device memory for the short plans of an ``AttnTransfer`` and those ``beside`` it, should they be needed on the device.
 
     A plan takes its place when it is made: a buffer that is allocated when a captured launch first needs it comes from
     the graph's private pool and can be the block of a temporary that was freed earlier in the capture, whose kernel every
     replay runs over the plan.  Places are of one size, cut off slabs, one slab at a time for each stream that plans are
     made for, and never given out twice.  A slab goes when the room and its last plan are gone, in the order of that stream.
-    Plan and launch of one layer of 333 tokens take 8.3 us, 8.2 without a place and 9.0 with a lock and places of the plans'
-    own sizes."""
+    Plan and launch of one layer of 333 tokens take 8.2 us, as without a place; 9.0 with a lock and places of the plans' own
+    sizes."""
 
     PLACES = 64         # of a slab, KVT_PLAN_IN_LAUNCH bytes each: 224 KiB
     STREAMS = 8         # most streams with a slab at hand
